@@ -25,7 +25,7 @@
 #include <vector>
 
 #include "../../include/geopvi_fwi2d.h"
-#include "fwi2d_kernels.cuh"
+#include "fwi2d_step_launch.h"
 #include "fwi2d_exact_adjoint.cuh"
 #include "fwi2d_pstd.cuh"
 
@@ -172,30 +172,60 @@ static void wavenumber(int ntx, int ntz, float dx, float dz, std::vector<float> 
         }
 }
 
-// Memory column of padded ix = 0.  The step kernel's 32-column tiles are
-// rim-only (no column in [Lc, ntx - Lc): zeros stored, no stencil), interior
-// (every column in [pml, ntx - pml): the lean sweep) or general (absorbing
-// strips: per-cell region tests and blends for the whole warp, about 2.5x
-// an interior tile).  The offset minimises that cost; the smallest wins ties.
+// How the step kernel tiles the columns when padded ix = 0 lies in memory
+// column xoff: 32-column units that hold a column of [c0, c1), the run of
+// them that are interior (every column in [pml, ntx - pml)), in pairs.
+static void column_units(int xoff, int c0, int c1, int ntx, int pml, int &unit0, int &units, int &wide0, int &wides)
+{
+    unit0 = (xoff + c0) / kTileX;
+    units = (xoff + c1 + kTileX - 1) / kTileX - unit0;
+    wide0 = std::min((xoff + pml + kTileX - 1) / kTileX, unit0 + units);
+    wides = std::max(0, (xoff + ntx - pml) / kTileX - wide0) / 2;
+}
+
+// Memory column of padded ix = 0: the one with the least work.  A narrow unit
+// costs about as much as two pairs (a blend per row, one column a lane).  The
+// smallest wins ties.
 static int column_offset(int ntx, int Lc, int pml)
 {
-    int best = 0;
-    long long best_cost = -1;
+    int best = 0, best_cost = -1;
     for (int xoff = 0; xoff < kTileX; ++xoff) {
-        const int tiles = (xoff + ntx + kTileX - 1) / kTileX;
-        long long cost = 0;
-        for (int t = 0; t < tiles; ++t) {
-            const int lo = t * kTileX - xoff, hi = lo + kTileX;
-            if (hi <= Lc || lo >= ntx - Lc) cost += 1;
-            else if (lo >= pml && hi <= ntx - pml) cost += 4;
-            else cost += 10;
-        }
+        int unit0, units, wide0, wides;
+        column_units(xoff, Lc, ntx - Lc, ntx, pml, unit0, units, wide0, wides);
+        const int cost = 2 * (units - 2 * wides) + wides;
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
             best = xoff;
         }
     }
     return best;
+}
+
+// 1/y^2 in two words (y the float divisor).
+static void inverse_square(float y, float *h, float *l)
+{
+    const double r = 1.0 / ((double)y * (double)y);
+    *h = (float)r;
+    *l = (float)(r - (double)*h);
+}
+
+// div2_two_least(y), or infinity where div_two is not exact for the divisor y;
+// cached, as the checks walk a binade.
+static float two_op_least(float y)
+{
+    static std::mutex m;
+    static std::map<uint32_t, float> cache;
+    uint32_t key;
+    std::memcpy(&key, &y, sizeof key);
+    {
+        std::lock_guard<std::mutex> lk(m);
+        auto it = cache.find(key);
+        if (it != cache.end()) return it->second;
+    }
+    const float least = two_op_exact(y) ? div2_two_least(y) : HUGE_VALF;
+    std::lock_guard<std::mutex> lk(m);
+    cache[key] = least;
+    return least;
 }
 
 static int derive(const gb_fwi2d_params &p, Derived &d)
@@ -231,8 +261,16 @@ static int derive(const gb_fwi2d_params &p, Derived &d)
     g.nt = p.nt;
     g.nti = p.nt_interval;
     g.nt_save = p.nt / p.nt_interval + ((p.nt % p.nt_interval) ? 1 : 0);
-    g.tiles_x = g.pitch / kTileX;
-    g.tiles_z = (g.ntz + kTileZ - 1) / kTileZ;
+    // A source or receiver in the rim writes to or samples cells that the step
+    // otherwise leaves out (validate() keeps both inside the padded grid).
+    auto in_rim = [](long long i, int n, int L) { return i < L || i >= n - L; };
+    const long long sx1 = g.s_ix0 + (long long)(g.ns - 1) * g.ds, rx1 = g.r_ix0 + (long long)(g.nr - 1) * g.dr;
+    const bool rim = in_rim(g.s_iz, g.ntz, g.Lc) || in_rim(g.r_iz, g.ntz, g.Lc) || in_rim(g.s_ix0, g.ntx, g.Lc) ||
+                     in_rim(sx1, g.ntx, g.Lc) || in_rim(g.r_ix0, g.ntx, g.Lc) || in_rim(rx1, g.ntx, g.Lc);
+    g.tile_r0 = rim ? 0 : g.Lc;
+    g.tile_r1 = rim ? g.ntz : g.ntz - g.Lc;
+    column_units(g.xoff, rim ? -g.xoff : g.Lc, rim ? g.pitch - g.xoff : g.ntx - g.Lc, g.ntx, g.pml, g.unit0, g.units,
+                 g.wide0, g.wides);
     g.fstride = (long long)g.ntz * g.pitch;
     g.pstride = (long long)g.nz * g.ipitch;
     g.dx = p.dx;
@@ -243,6 +281,14 @@ static int derive(const gb_fwi2d_params &p, Derived &d)
     g.rdz = 1.0f / p.dz;
     g.fast_dx = division_is_exact(p.dx) ? 1 : 0;
     g.fast_dz = division_is_exact(p.dz) ? 1 : 0;
+    const float least_x = two_op_least(p.dx), least_z = two_op_least(p.dz);
+    g.lo1 = least_x < HUGE_VALF ? kDivLo : HUGE_VALF;
+    g.lo2 = std::max(least_x, least_z);
+    g.two = g.lo2 < HUGE_VALF ? 1 : 0;
+    reciprocal_pair(p.dx, &g.rxh, &g.rxl);
+    reciprocal_pair(p.dz, &g.rzh, &g.rzl);
+    inverse_square(p.dx, &g.x2h, &g.x2l);
+    inverse_square(p.dz, &g.z2h, &g.z2l);
     ricker(p.nt, p.dt, p.f0, d.rik);
     g.pstd = p.laplace_solver == 1 ? 1 : 0;
     if (g.pstd) wavenumber(g.ntx, g.ntz, p.dx, p.dz, d.kk);
@@ -301,7 +347,7 @@ static Layout plan_layout_exact(const Geom &g, int nsamples, int resident, bool 
     L.ckpt_nseg = (g.nt + L.ckpt_k - 1) / L.ckpt_k;
     const size_t field = sizeof(float) * g.fstride;
     size_t off = 0;
-    L.status = off; off = align256(off + sizeof(int));
+    L.status = off; off = align256(off + kStatusWords * sizeof(int));
     L.vdt = off;    off = align256(off + field * nsamples);
     L.ring = off;   off = align256(off + field * 3 * resident);
     L.ckpt = off;
@@ -336,7 +382,7 @@ static Layout plan_layout(const Geom &g, int nsamples, int resident, bool syn_in
         snaps = L.ckpt_k / g.nti;
     }
     size_t off = 0;
-    L.status = off; off = align256(off + sizeof(int));
+    L.status = off; off = align256(off + kStatusWords * sizeof(int));
     L.vdt = off;   off = align256(off + sizeof(float) * g.fstride * nsamples);
     L.ring = off;  off = align256(off + sizeof(float) * g.fstride * 3 * resident);
     if (checkpoint) {
@@ -364,8 +410,9 @@ static Layout plan_layout(const Geom &g, int nsamples, int resident, bool syn_in
 
 // Padded v*dt for every sample: get_velp's replication (a clamp) times dt,
 // the float product that powf(v*dt, 2) and s = v*dt/dx start from.
-__global__ void k_prepare(const Geom g, const float *__restrict__ vel, float *__restrict__ vdt,
-                          int nsamples)
+// status[1] is set where a velocity's (v dt)^2 is not finite.
+__global__ void k_prepare(const Geom g, const float *__restrict__ vel, float *__restrict__ vdt, int nsamples,
+                          int *__restrict__ status)
 {
     const long long total = (long long)nsamples * g.fstride;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
@@ -377,6 +424,7 @@ __global__ void k_prepare(const Geom g, const float *__restrict__ vel, float *__
         float v = 0.0f;
         if (ix >= 0 && ix < g.ntx)
             v = fm(padded_velocity(g, vel + (long long)s * g.nx * g.nz, iz, ix), g.dt);
+        if (!isfinite(fm(v, v))) atomicOr(status + 1, 1);
         vdt[e] = v;
     }
 }
@@ -577,10 +625,6 @@ static bool make_map(CUtensorMap &m, void *base, const Geom &g, long long depth,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-struct Maps {
-    CUtensorMap p1;
-};
-
 // First failure status of the launches being enqueued on this thread.
 static thread_local int t_enqueue_error = 0;
 
@@ -621,46 +665,28 @@ static const SideStream *side_stream(bool create)
 // one half's launches overlap the other half's work.
 constexpr int kSplitMinResident = 32;
 
-static bool make_maps(Maps &m, const Geom &g, float *ring, int resident)
+// The step kernel's maps over `fields` padded fields, boxes of the variant's tiles.
+static bool make_step_maps(StepMaps &m, void *base, const Geom &g, long long fields, int variant)
 {
-    return make_map(m.p1, ring, g, 3LL * resident, kBoxX, kTileZ + 2 * (g.Lc - 1));
+    const int H = g.Lc - 1, rows = kStepVariants[variant].rows + 2 * H;
+    return make_map(m.narrow, base, g, fields, step_box_x(H, false), rows) &&
+           make_map(m.wide, base, g, fields, step_box_x(H, true), rows);
 }
 
-// overlap: the previous operation on `st` is the step before this one, and
-// this step may be launched programmatically (its blocks become resident
-// while that step drains; k_step waits on it before any global access).
-template <int H, int U, int MINB>
-static void launch_step_variant(bool adj, const Maps &m, const Geom &g, const Batch &b, int nres,
-                                const StepArgs &sa, cudaStream_t st, bool overlap)
+// The step kernel's variant for launches of `nres` solves of this grid: the
+// tallest tiles that still give the device's 152 x 28 resident warps enough to
+// do.  Tall tiles share their halo rows; short ones shorten the chain of rows
+// that a small launch waits for.  Misfit + gradient, us per step with 16 / 8 /
+// 4 / 2 rows (800 steps): 160 solves of 200x400 (25600 tiles of 16 rows) 76 /
+// 89 / 113 / 178, 16 of 400x800 (7728) 23.1 / 22.4 / 31.8 / 58.2, 40 of
+// 200x400 (6400; 11360 of 8 rows) 21.1 / 18.2 / 24.1 / 43.8, 20 of 200x400
+// (5680 of 8) 17.6 / 13.3 / 13.5 / 22.8, 12 of 110x250 (2664 of 4) 14.0 / 10.3
+// / 7.8 / 6.8, 2 of 32x48 9.4 / 7.8 / 4.8 / 3.3.
+static int step_variant_for(const Geom &g, long long nres)
 {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nres, g.tiles_x * g.tiles_z);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = TileShape<H>::kSmem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
-    const cudaError_t e = adj ? cudaLaunchKernelEx(&cfg, k_step<H, true, U, MINB>, m.p1, g, b, sa)
-                              : cudaLaunchKernelEx(&cfg, k_step<H, false, U, MINB>, m.p1, g, b, sa);
-    if (e != cudaSuccess) t_enqueue_error = GB_FWI2D_ECUDA;
-}
-
-template <int H>
-static void launch_step(bool adj, const Maps &m, const Geom &g, const Batch &b, int nres,
-                        const StepArgs &sa, cudaStream_t st, int variant, bool overlap)
-{
-    static_assert(kNumStepVariants == 4, "one case per entry of kStepVariants");
-    constexpr StepVariant v1 = kStepVariants[1], v2 = kStepVariants[2], v3 = kStepVariants[3],
-                          v0 = kStepVariants[0];
-    switch (variant) {
-    case 1: launch_step_variant<H, v1.rows, v1.min_blocks>(adj, m, g, b, nres, sa, st, overlap); break;
-    case 2: launch_step_variant<H, v2.rows, v2.min_blocks>(adj, m, g, b, nres, sa, st, overlap); break;
-    case 3: launch_step_variant<H, v3.rows, v3.min_blocks>(adj, m, g, b, nres, sa, st, overlap); break;
-    default: launch_step_variant<H, v0.rows, v0.min_blocks>(adj, m, g, b, nres, sa, st, overlap); break;
-    }
+    if (nres * step_tiles(g, 16) >= 7300) return 0;
+    if (nres * step_tiles(g, 8) >= 5000) return 1;
+    return nres * step_tiles(g, 4) >= 5000 ? 2 : 3;
 }
 
 // ---------------------------------------------------------------------------
@@ -785,16 +811,18 @@ static int step_pstd(bool adj, const Geom &g, const Batch &b, int nres, const St
 }
 
 // One time step of the wave; returns the number of this library's kernels.
-static int step(bool adj, const Maps &m, const Geom &g, const Batch &b, int nres, const StepArgs &sa,
+static int step(bool adj, const StepMaps &m, const Geom &g, const Batch &b, int nres, const StepArgs &sa,
                 cudaStream_t st, int variant, bool overlap = false)
 {
     if (g.pstd) return step_pstd(adj, g, b, nres, sa, st);
+    cudaError_t e;
     switch (g.Lc - 1) {
-    case 3: launch_step<3>(adj, m, g, b, nres, sa, st, variant, overlap); break;
-    case 4: launch_step<4>(adj, m, g, b, nres, sa, st, variant, overlap); break;
-    case 5: launch_step<5>(adj, m, g, b, nres, sa, st, variant, overlap); break;
-    default: launch_step<6>(adj, m, g, b, nres, sa, st, variant, overlap); break;
+    case 3: e = launch_step_h<3>(adj, m, g, b, nres, sa, st, variant, overlap); break;
+    case 4: e = launch_step_h<4>(adj, m, g, b, nres, sa, st, variant, overlap); break;
+    case 5: e = launch_step_h<5>(adj, m, g, b, nres, sa, st, variant, overlap); break;
+    default: e = launch_step_h<6>(adj, m, g, b, nres, sa, st, variant, overlap); break;
     }
+    if (e != cudaSuccess) t_enqueue_error = GB_FWI2D_ECUDA;
     return 1;
 }
 
@@ -809,18 +837,13 @@ struct Call {
     unsigned flags;
     char *work;
     bool profile;
-    Maps maps;
-    Maps maps2;  // checkpointing: the adjoint's ring; exact gradient: the store
-    Maps maps3;  // exact gradient: nu beside the adjoint levels
+    StepMaps maps;
+    StepMaps maps2;     // checkpointing: the adjoint's ring; exact gradient: the store
+    CUtensorMap adj_nu, adj_store;  // exact gradient: nu beside the adjoint levels, the store
     const float *kk = nullptr;  // pseudo-spectral mode: |k|^2 table on the device
     int variant = 0;            // k_step variant (kStepVariants)
     bool single_stream = false; // never fork onto the side stream (no stream or event is created)
     bool clear_status = true;   // zero the status word first (false: keep an earlier call's flags)
-    // Tuning: waves [0, trials.size()) run variant trials[i] between events
-    // trial_ev[i]; later waves run `variant`.
-    std::vector<int> trials;
-    std::vector<std::pair<cudaEvent_t, cudaEvent_t>> trial_ev;
-    int wave_variant(long long wave) const { return wave < (long long)trials.size() ? trials[wave] : variant; }
 };
 
 static int grid_for(long long n, int threads)
@@ -863,10 +886,12 @@ static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStre
     // forward: data only, checkpoints at segment starts
     b.ring = ring;
     b.store = 0;
-    cudaMemset2DAsync(ring, ring_pitch, 0, 2 * fbytes, nres, st);
+    cudaMemsetAsync(ring, 0, ring_pitch * nres, st);  // all three levels: the steps leave the rim's zeros
     profile_span(e0, e1);
+    bool prev_step = false;  // the last operation enqueued on st is a step
     for (int k = 0; k < g.nt; ++k) {
         if (k % K == 0) {
+            prev_step = false;
             const int s = k / K;
             cudaMemcpy2DAsync((char *)ck + (size_t)2 * s * fbytes, ck_pitch, (char *)ring + (size_t)(k % 3) * fbytes,
                               ring_pitch, fbytes, nres, cudaMemcpyDeviceToDevice, st);
@@ -875,12 +900,13 @@ static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStre
                               cudaMemcpyDeviceToDevice, st);
         }
         const StepArgs sa = ring_step(k, k, -1, c.d->rik[k]);
-        launches += step(false, c.maps, g, b, nres, sa, st, c.variant);
+        launches += step(false, c.maps, g, b, nres, sa, st, c.variant, prev_step);
+        prev_step = true;
     }
     close_span(e0, e1, g.nt);
 
     // adjoint, segment by segment from the last
-    cudaMemset2DAsync(ring2, ring_pitch, 0, 2 * fbytes, nres, st);
+    cudaMemsetAsync(ring2, 0, ring_pitch * nres, st);
     Batch ba = b;
     ba.ring = ring2;
     b.store = 1;
@@ -892,13 +918,17 @@ static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStre
         cudaMemcpy2DAsync((char *)ring + (size_t)((k0 + 1) % 3) * fbytes, ring_pitch,
                           (char *)ck + (size_t)(2 * s + 1) * fbytes, ck_pitch, fbytes, nres,
                           cudaMemcpyDeviceToDevice, st);
+        prev_step = false;
         for (int k = k0; k < k1; ++k) {  // recompute the segment's forward steps, storing them
             const StepArgs sa = ring_step(k, k, (k % g.nti) == 0 ? k / g.nti - snap0 : -1, c.d->rik[k]);
-            launches += step(false, c.maps, g, b, nres, sa, st, c.variant);
+            launches += step(false, c.maps, g, b, nres, sa, st, c.variant, prev_step);
+            prev_step = true;
         }
         for (int it = k1 - 1; it >= k0; --it) {  // the segment's adjoint steps
-            const StepArgs sa = ring_step(g.nt - 1 - it, it, (it % g.nti) == 0 ? it / g.nti - snap0 : -1, 0.0f);
-            launches += step(true, c.maps2, g, ba, nres, sa, st, c.variant);
+            const int k = g.nt - 1 - it;
+            StepArgs sa = ring_step(k, it, (it % g.nti) == 0 ? it / g.nti - snap0 : -1, 0.0f);
+            adjoint_terms(sa, g.nti, k, g.nt - k1, g.nt - 1 - k0, snap0);
+            launches += step(true, c.maps2, g, ba, nres, sa, st, c.variant, prev_step);
         }
     }
     close_span(e0, e1, 2LL * g.nt);
@@ -914,7 +944,7 @@ static void launch_adjoint_exact(const Call &c, const ExactBatch &x, int nres, i
 {
     const Geom &g = c.d->g;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(g.tiles_x * g.tiles_z), nres);
+    cfg.gridDim = dim3((unsigned)(g.pitch / kTileX * ((g.ntz + kTileZ - 1) / kTileZ)), nres);
     cfg.blockDim = dim3(kAdjThreads);
     cfg.dynamicSmemBytes = AdjShape<H>::kSmem;
     cfg.stream = st;
@@ -923,7 +953,7 @@ static void launch_adjoint_exact(const Call &c, const ExactBatch &x, int nres, i
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = overlap ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, k_adjoint_tile<H>, c.maps3.p1, c.maps2.p1, g, x, k, lev1, rik) != cudaSuccess)
+    if (cudaLaunchKernelEx(&cfg, k_adjoint_tile<H>, c.adj_nu, c.adj_store, g, x, k, lev1, rik) != cudaSuccess)
         t_enqueue_error = GB_FWI2D_ECUDA;
 }
 
@@ -965,14 +995,14 @@ static long long enqueue_exact(const Call &c, cudaStream_t st)
     const size_t fbytes = sizeof(float) * g.fstride;
     const size_t ring_pitch = 3 * fbytes, store_pitch = (size_t)levels * fbytes, ck_pitch = 2 * (size_t)nseg * fbytes;
 
-    k_prepare<<<grid_for((long long)c.nsamples * g.fstride, 256), 256, 0, st>>>(g, c.vel, vdt, c.nsamples);
+    if (c.clear_status) cudaMemsetAsync(status, 0, kStatusWords * sizeof(int), st);
+    k_prepare<<<grid_for((long long)c.nsamples * g.fstride, 256), 256, 0, st>>>(g, c.vel, vdt, c.nsamples, status);
     float *abeta = (float *)(c.work + L.abeta);
     int4 *cells = (int4 *)(c.work + L.cells);
     float *taps = (float *)(c.work + L.taps);
     k_exact_tables<<<grid_for((long long)c.nsamples * g.fstride, 256), 256, 0, st>>>(g, c.tab.coef, vdt, c.nsamples,
                                                                                    cells, abeta, taps);
     launches += 2;
-    if (c.clear_status) cudaMemsetAsync(status, 0, sizeof(int), st);
     cudaMemsetAsync(gpad, 0, fbytes * ninst, st);
 
     Batch b{};
@@ -1021,6 +1051,9 @@ static long long enqueue_exact(const Call &c, cudaStream_t st)
         prev_step = true;
     };
     const int wave = (c.flags & GB_FWI2D_PLAIN) ? 1 : L.resident;
+    // The steps leave the rim of the levels they write as it is: zero, once
+    // for all waves (later writes to a level never touch its rim).
+    cudaMemsetAsync(store, 0, store_pitch * std::min<long long>(wave, ninst), st);
     for (long long i0 = 0; i0 < ninst; i0 += wave) {
         const int nres = (int)std::min<long long>(wave, ninst - i0);
         b.inst0 = bs.inst0 = x.inst0 = (int)i0;
@@ -1029,7 +1062,7 @@ static long long enqueue_exact(const Call &c, cudaStream_t st)
             cudaMemset2DAsync(store, store_pitch, 0, 2 * fbytes, nres, st);
             for (int it = 0; it < g.nt; ++it) fwd_store(it, it, nres);
         } else {
-            cudaMemset2DAsync(ring, ring_pitch, 0, 2 * fbytes, nres, st);
+            cudaMemsetAsync(ring, 0, ring_pitch * nres, st);
             for (int it = 0; it < g.nt; ++it) {
                 if (it % K == 0) {
                     const int s = it / K;  // the step's (p0, p1) = (P^{it-1}, P^it)
@@ -1095,10 +1128,9 @@ static long long enqueue(const Call &c, cudaStream_t st)
     const bool fwd_only = (c.flags & GB_FWI2D_FORWARD_ONLY) != 0;
     const long long ninst = (long long)c.nsamples * g.ns;
 
-    k_prepare<<<grid_for((long long)c.nsamples * g.fstride, 256), 256, 0, st>>>(g, c.vel, vdt,
-                                                                                c.nsamples);
+    if (c.clear_status) cudaMemsetAsync(status, 0, kStatusWords * sizeof(int), st);
+    k_prepare<<<grid_for((long long)c.nsamples * g.fstride, 256), 256, 0, st>>>(g, c.vel, vdt, c.nsamples, status);
     ++launches;
-    if (c.clear_status) cudaMemsetAsync(status, 0, sizeof(int), st);
     if (!fwd_only) cudaMemsetAsync(gacc, 0, sizeof(float) * g.pstride * ninst, st);
 
     Batch b;
@@ -1120,7 +1152,7 @@ static long long enqueue(const Call &c, cudaStream_t st)
     b.slot0 = 0;
     b.levels = 3;
     b.tm_slot0 = 0;
-    const Maps &maps = c.maps;
+    const StepMaps &maps = c.maps;
 
     const int wave = plain ? 1 : c.L.resident;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1132,24 +1164,16 @@ static long long enqueue(const Call &c, cudaStream_t st)
     for (long long i0 = 0; i0 < ninst && ckpt; i0 += wave) {
         const int nres = (int)std::min<long long>(wave, ninst - i0);
         b.inst0 = (int)i0;
-        const long long wi = i0 / wave;
-        Call cw = c;
-        cw.variant = c.wave_variant(wi);
-        if (wi < (long long)c.trials.size()) cudaEventRecord(c.trial_ev[wi].first, st);
-        launches += enqueue_checkpointed(cw, b, nres, st);
-        if (wi < (long long)c.trials.size()) cudaEventRecord(c.trial_ev[wi].second, st);
+        launches += enqueue_checkpointed(c, b, nres, st);
     }
     for (long long i0 = 0; i0 < ninst && !ckpt; i0 += wave) {
         const int nres = (int)std::min<long long>(wave, ninst - i0);
         b.inst0 = (int)i0;
-        const long long wi = i0 / wave;
-        const int variant = c.wave_variant(wi);
-        if (wi < (long long)c.trials.size()) cudaEventRecord(c.trial_ev[wi].first, st);
         for (int pass = 0; pass < (fwd_only ? 1 : 2); ++pass) {
             const bool adj = pass == 1;
-            // p0 and p1 of step 0 start at zero (wavefield_initialization).
-            cudaMemset2DAsync(ring, sizeof(float) * 3 * g.fstride, 0, sizeof(float) * 2 * g.fstride,
-                              nres, st);
+            // p0 and p1 of step 0 start at zero (wavefield_initialization), and
+            // the third level too: the steps leave the rim as it is.
+            cudaMemsetAsync(ring, 0, sizeof(float) * 3 * g.fstride * nres, st);
             cudaEvent_t e0 = nullptr, e1 = nullptr;
             if (c.profile && cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess)
                 cudaEventRecord(e0, st);
@@ -1163,9 +1187,10 @@ static long long enqueue(const Call &c, cudaStream_t st)
             }
             for (int k = 0; k < g.nt; ++k) {
                 const int it = adj ? g.nt - 1 - k : k;
-                const StepArgs sa = ring_step(k, it, (it % g.nti) == 0 ? it / g.nti : -1, adj ? 0.0f : c.d->rik[it]);
-                launches += step(adj, maps, g, b, nlo, sa, st, variant, k > 0);
-                if (split) launches += step(adj, maps, g, bhi, nres - nlo, sa, side->s, variant, k > 0);
+                StepArgs sa = ring_step(k, it, (it % g.nti) == 0 ? it / g.nti : -1, adj ? 0.0f : c.d->rik[it]);
+                if (adj) adjoint_terms(sa, g.nti, k, 0, g.nt - 1, 0);
+                launches += step(adj, maps, g, b, nlo, sa, st, c.variant, k > 0);
+                if (split) launches += step(adj, maps, g, bhi, nres - nlo, sa, side->s, c.variant, k > 0);
             }
             if (split) {  // join
                 cudaEventRecord(side->join, side->s);
@@ -1177,7 +1202,6 @@ static long long enqueue(const Call &c, cudaStream_t st)
                 t_profile.launches += g.nt;
             }
         }
-        if (wi < (long long)c.trials.size()) cudaEventRecord(c.trial_ev[wi].second, st);
     }
     if (c.grad && !fwd_only) {
         k_reduce_grad<<<grid_for((long long)c.nsamples * g.nz * g.nx, 256), 256, 0, st>>>(
@@ -1231,6 +1255,7 @@ struct FusedPiece {
 struct FusedLaunch {
     std::vector<int> pieces;  // indices into the wave's pieces, longest nt first
     int maxnt = 0;
+    int variant = 0;          // the step kernel's variant (tile rows)
     MultiArgs args;           // the launch's parameter (the first half of its solves when split)
     bool split = false;       // the second half runs as its own launch on the side stream
     MultiArgs args_hi;
@@ -1239,13 +1264,12 @@ struct FusedLaunch {
 // Split a launch's table at solve `at` (among its tm_slot0 order): solves
 // below stay, the rest move to `hi` -- a piece that straddles `at` is cut in
 // two.  Each half's first blocks start again at 0.
-static void split_args(MultiArgs &lo, MultiArgs &hi, int at, const Geom &g, bool fwd_only)
+static void split_args(MultiArgs &lo, MultiArgs &hi, int at, const Geom &g, bool fwd_only, int tiles)
 {
     MultiArgs all = lo;
     hi = all;
     lo.npieces = hi.npieces = 0;
     int blo = 0, bhi = 0;
-    const int tiles = g.tiles_x * g.tiles_z;
     for (int q = 0; q < all.npieces; ++q) {
         const PieceArgs &pc = all.piece[q];
         const int s0 = pc.tm_slot0, s1 = pc.tm_slot0 + pc.nres;
@@ -1286,7 +1310,7 @@ struct FusedWave {
 static std::vector<long long> grid_key(const Geom &g)
 {
     std::vector<long long> k = {g.ntx, g.ntz, g.pitch, g.xoff, g.nx, g.nz, g.ipitch, g.ioff, g.pml, g.Lc, g.pml0,
-                                g.tiles_x, g.tiles_z, g.fast_dx, g.fast_dz, g.pstd, g.fstride, g.pstride};
+                                g.tile_r0, g.tile_r1, g.unit0, g.units, g.wide0, g.wides, g.fast_dx, g.fast_dz, g.pstd, g.fstride, g.pstride};
     uint32_t u;
     for (float f : {g.dx, g.dz, g.dt, g.rdx, g.rdz, g.fd[0], g.fd[1], g.fd[2], g.fd[3], g.fd[4], g.fd[5], g.fd[6],
                     g.fd[7]}) {
@@ -1440,50 +1464,6 @@ static int plan_instances(const gb_fwi2d_instance *inst, int n, unsigned flags, 
     return close();
 }
 
-template <int H, int NP>
-static void launch_multi_np(bool adj, const MultiArgs &full, int nact, int k, cudaStream_t st, bool overlap)
-{
-    constexpr StepVariant v = kStepVariants[0];
-    MultiArgsN<NP> a;
-    a.tm = full.tm;
-    a.gc = full.gc;
-    a.coef = full.coef;
-    a.status = full.status;
-    a.blend_fp32 = full.blend_fp32;
-    a.imaging = full.imaging;
-    a.store = full.store;
-    a.npieces = full.npieces;
-    for (int q = 0; q <= NP; ++q) a.first[q] = full.first[q];
-    for (int q = 0; q < NP; ++q) a.piece[q] = full.piece[q];
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)full.first[nact]);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = TileShape<H>::kSmem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
-    const cudaError_t e =
-        adj ? cudaLaunchKernelEx(&cfg, k_step_multi<H, true, v.rows, v.min_blocks, NP>, a, nact, k)
-            : cudaLaunchKernelEx(&cfg, k_step_multi<H, false, v.rows, v.min_blocks, NP>, a, nact, k);
-    if (e != cudaSuccess) t_enqueue_error = GB_FWI2D_ECUDA;
-}
-
-// The smallest parameter table that holds the launch's pieces.
-template <int H>
-static void launch_multi(bool adj, const MultiArgs &args, int nact, int k, cudaStream_t st, bool overlap)
-{
-    static_assert(kMaxPieces == 16, "tables of 1, 4 and 16 pieces");
-    if (args.npieces <= 1)
-        launch_multi_np<H, 1>(adj, args, nact, k, st, overlap);
-    else if (args.npieces <= 4)
-        launch_multi_np<H, 4>(adj, args, nact, k, st, overlap);
-    else
-        launch_multi_np<H, 16>(adj, args, nact, k, st, overlap);
-}
-
 // Enqueue one chunk (instances of one FD order, grouped by grid, longest nt
 // first) laid out as: the status word, the instances' kept buffers (Ricker
 // tables first: they are copied from the host in one transfer), then one wave
@@ -1544,6 +1524,10 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
             std::memset(&A, 0, sizeof A);
             const size_t base = wave_base + used;
             int slots = 0, blocks = 0;
+            for (int j : l.pieces) slots += w.pieces[j].r;
+            l.variant = step_variant_for(g0, slots);
+            const int tiles = step_tiles(g0, kStepVariants[l.variant].rows);
+            slots = 0;
             for (size_t q = 0; q < l.pieces.size(); ++q) {
                 FusedPiece &pc = w.pieces[l.pieces[q]];
                 const FusedInst &f = fi[pc.inst];
@@ -1574,7 +1558,7 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
                 P.first_block = blocks;
                 A.first[q] = blocks;
                 slots += pc.r;
-                blocks += pc.r * g.tiles_x * g.tiles_z;
+                blocks += pc.r * tiles;
             }
             A.first[l.pieces.size()] = blocks;
             used = align256(used + sizeof(float) * g0.fstride * 3 * slots);
@@ -1585,7 +1569,7 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
                 A.piece[q].psave = (float *)(work + pc.psave);
                 if (!fwd_only) used = align256(used + sizeof(float) * g.pstride * g.nt_save * pc.r);
             }
-            if (!make_map(A.tm, work + base, g0, 3LL * slots, kBoxX, kTileZ + 2 * (g0.Lc - 1))) return -1;
+            if (!make_step_maps(A.tm, work + base, g0, 3LL * slots, l.variant)) return -1;
             A.gc = g0;
             A.coef = f0.tab.coef;
             A.status = status;
@@ -1596,7 +1580,7 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
             // Launches of at least kSplitMinResident solves run as two halves on
             // two streams, so the tail of one half's step overlaps the other's.
             l.split = side != nullptr && slots >= kSplitMinResident;
-            if (l.split) split_args(A, l.args_hi, slots / 2, g0, fwd_only);
+            if (l.split) split_args(A, l.args_hi, slots / 2, g0, fwd_only, tiles);
         }
     }
     // From pageable memory: the copy has taken the host image when it returns.
@@ -1604,22 +1588,21 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
         cudaMemcpyAsync(work + kFusedHeader, host.data(), host.size(), cudaMemcpyHostToDevice, st) != cudaSuccess)
         return -1;
     long long launches = 0;
-    if (clear_status) cudaMemsetAsync(status, 0, sizeof(int), st);
+    if (clear_status) cudaMemsetAsync(status, 0, kStatusWords * sizeof(int), st);
     for (const auto &f : fi) {
         const Geom &g = f.d.g;
         k_prepare<<<grid_for((long long)f.x->nsamples * g.fstride, 256), 256, 0, st>>>(g, f.x->vel,
                                                                                      (float *)(work + f.vdt),
-                                                                                     f.x->nsamples);
+                                                                                     f.x->nsamples, status);
         ++launches;
         if (!fwd_only) cudaMemsetAsync(work + f.gacc, 0, sizeof(float) * g.pstride * f.ninst, st);
     }
     for (const auto &w : waves) {
         for (int pass = 0; pass < (fwd_only ? 1 : 2); ++pass) {
             const bool adj = pass == 1;
-            for (const auto &pc : w.pieces) {  // p0 and p1 of step 0 start at zero (wavefield_initialization)
+            for (const auto &pc : w.pieces) {  // the rings start at zero (wavefield_initialization), their rims stay so
                 const Geom &g = fi[pc.inst].d.g;
-                cudaMemset2DAsync(work + pc.ring, sizeof(float) * 3 * g.fstride, 0, sizeof(float) * 2 * g.fstride,
-                                  pc.r, st);
+                cudaMemsetAsync(work + pc.ring, 0, sizeof(float) * 3 * g.fstride * pc.r, st);
             }
             cudaEvent_t e0 = nullptr, e1 = nullptr;
             if (profile && cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess)
@@ -1638,23 +1621,25 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
             // Each step waits for the launch before it on its stream; the first
             // of a pass on each stream follows the rings' reset and launches normally.
             bool started = false, started_hi = false;
-            auto launch = [&](const MultiArgs &a, int &na, int k, cudaStream_t s, bool &on) {
+            auto launch = [&](const MultiArgs &a, int &na, int k, cudaStream_t s, bool &on, int variant) {
                 while (na > 0 && a.piece[na - 1].nt <= k) --na;  // the pieces still running: a prefix
                 if (na == 0) return;
+                cudaError_t e;
                 switch (H) {
-                case 3: launch_multi<3>(adj, a, na, k, s, on); break;
-                case 4: launch_multi<4>(adj, a, na, k, s, on); break;
-                case 5: launch_multi<5>(adj, a, na, k, s, on); break;
-                default: launch_multi<6>(adj, a, na, k, s, on); break;
+                case 3: e = launch_multi_h<3>(adj, a, na, k, s, variant, on); break;
+                case 4: e = launch_multi_h<4>(adj, a, na, k, s, variant, on); break;
+                case 5: e = launch_multi_h<5>(adj, a, na, k, s, variant, on); break;
+                default: e = launch_multi_h<6>(adj, a, na, k, s, variant, on); break;
                 }
+                if (e != cudaSuccess) t_enqueue_error = GB_FWI2D_ECUDA;
                 on = true;
                 ++launches;
             };
             for (int k = 0; k < w.maxnt; ++k) {
                 for (size_t li = 0; li < w.launches.size(); ++li) {
                     const FusedLaunch &l = w.launches[li];
-                    launch(l.args, nact[li], k, st, started);
-                    if (l.split) launch(l.args_hi, nact_hi[li], k, side->s, started_hi);
+                    launch(l.args, nact[li], k, st, started, l.variant);
+                    if (l.split) launch(l.args_hi, nact_hi[li], k, side->s, started_hi, l.variant);
                 }
             }
             if (forked) {  // join
@@ -1713,77 +1698,22 @@ static std::vector<long long> graph_key(const Call &c, int dev)
     return k;
 }
 
-// ---------------------------------------------------------------------------
-// Variant tuner.  Every k_step variant computes the same values bit for bit,
-// so the caller's own work serves as trials: while a (geometry, batch size,
-// wave size, mode) has untried variants, each wave of a call runs one of them
-// between two events (a six-wave batch tries all four in its first call);
-// later calls read the finished timings -- polled, never waited for -- and
-// run the fastest.  Calls with trials run eagerly; graph capture starts once
-// the choice is made.
-// ---------------------------------------------------------------------------
-struct TuneState {
-    bool measured[kNumStepVariants] = {};
-    bool inflight[kNumStepVariants] = {};
-    float ms[kNumStepVariants] = {};
-    cudaEvent_t e0[kNumStepVariants] = {}, e1[kNumStepVariants] = {};
-    int best = 0;  // fastest measured (the default until one is measured)
-    bool done = false;
-};
-static std::mutex g_tune_mutex;
-static std::map<std::vector<long long>, TuneState> g_tune;
-
-static std::vector<long long> tune_key(const Geom &g, int nsamples, int resident, unsigned flags, int dev)
+// The tensor maps of a call's workspace (the pseudo-spectral step reads the
+// ring directly).
+static bool make_call_maps(Call &c, const Geom &g, const Layout &L, unsigned flags)
 {
-    std::vector<long long> k{dev, nsamples, resident,
-                             (long long)(flags & (GB_FWI2D_IMAGING | GB_FWI2D_PLAIN | GB_FWI2D_CHECKPOINT |
-                                                  GB_FWI2D_FORWARD_ONLY | GB_FWI2D_EXACT_GRADIENT))};
-    const int *gi = (const int *)&g;
-    for (size_t i = 0; i < sizeof(Geom) / sizeof(int); ++i) k.push_back(gi[i]);
-    return k;
-}
-
-// Read the trials whose events have completed (g_tune_mutex held).
-static void tune_harvest(TuneState &t)
-{
-    bool all = true;
-    for (int v = 0; v < kNumStepVariants; ++v) {
-        if (t.inflight[v] && cudaEventQuery(t.e1[v]) == cudaSuccess) {
-            float ms = 0.0f;
-            // An unreadable timing counts as measured and never wins.
-            t.ms[v] = cudaEventElapsedTime(&ms, t.e0[v], t.e1[v]) == cudaSuccess ? ms : 3.4e38f;
-            t.measured[v] = true;
-            t.inflight[v] = false;
-        }
-        all = all && t.measured[v];
+    if (g.pstd) return true;
+    if (!make_step_maps(c.maps, c.work + L.ring, g, 3LL * L.resident, c.variant)) return false;
+    if (flags & GB_FWI2D_FORWARD_ONLY) return true;
+    if (flags & GB_FWI2D_EXACT_GRADIENT) {
+        const long long levels = (long long)(L.ckpt_k + 2) * L.resident;
+        const int box_z = kTileZ + 2 * (g.Lc - 1);
+        return make_step_maps(c.maps2, c.work + L.store, g, levels, c.variant) &&
+               make_map(c.adj_store, c.work + L.store, g, levels, kBoxX, box_z) &&
+               make_map(c.adj_nu, c.work + L.nu, g, 3LL * L.resident, kBoxX, box_z);
     }
-    int best = -1;
-    for (int v = 0; v < kNumStepVariants; ++v)
-        if (t.measured[v] && (best < 0 || t.ms[v] < t.ms[best])) best = v;
-    if (best >= 0) t.best = best;
-    t.done = all;
-}
-
-// The calling batch's plan: trial variants for its first waves (with their
-// events) and the variant for the rest.
-static void tune_plan(const std::vector<long long> &key, long long nwaves, Call &c)
-{
-    std::lock_guard<std::mutex> lk(g_tune_mutex);
-    TuneState &t = g_tune[key];
-    tune_harvest(t);
-    c.variant = t.best;
-    if (t.done) return;
-    for (int v = 0; v < kNumStepVariants && (long long)c.trials.size() < nwaves; ++v) {
-        if (t.measured[v] || t.inflight[v]) continue;
-        if (!t.e0[v] && (cudaEventCreate(&t.e0[v]) != cudaSuccess || cudaEventCreate(&t.e1[v]) != cudaSuccess)) {
-            t.measured[v] = true;  // no events: leave this variant out
-            t.ms[v] = 3.4e38f;
-            continue;
-        }
-        t.inflight[v] = true;
-        c.trials.push_back(v);
-        c.trial_ev.emplace_back(t.e0[v], t.e1[v]);
-    }
+    return !(flags & GB_FWI2D_CHECKPOINT) ||
+           make_step_maps(c.maps2, c.work + L.ring2, g, 3LL * L.resident, c.variant);
 }
 
 static int run_graph(const Call &c, cudaStream_t st, long long &launches)
@@ -1918,19 +1848,10 @@ static int batch_impl(const gb_fwi2d_params *p, int nsamples, const float *vel, 
     c.work = (char *)work;
     c.profile = (flags & GB_FWI2D_PROFILE) && !(flags & GB_FWI2D_GRAPH);
     c.clear_status = clear_status;
-    // The step kernel's tensor maps (the pseudo-spectral step reads the ring directly).
-    if (!d.g.pstd && !make_maps(c.maps, d.g, (float *)(c.work + L.ring), L.resident))
-        return GB_FWI2D_ECUDA;
-    if (ckpt && !exact && !d.g.pstd && !(flags & GB_FWI2D_FORWARD_ONLY) &&
-        !make_maps(c.maps2, d.g, (float *)(c.work + L.ring2), L.resident))
-        return GB_FWI2D_ECUDA;
-    if (exact && !d.g.pstd && !(flags & GB_FWI2D_FORWARD_ONLY)) {  // the store and nu, as the step's tiles
-        const int box_z = kTileZ + 2 * (d.g.Lc - 1);
-        if (!make_map(c.maps2.p1, (float *)(c.work + L.store), d.g, (long long)(L.ckpt_k + 2) * L.resident, kBoxX,
-                      box_z) ||
-            !make_map(c.maps3.p1, (float *)(c.work + L.nu), d.g, 3LL * L.resident, kBoxX, box_z))
-            return GB_FWI2D_ECUDA;
-    }
+    const unsigned forced = (flags >> GB_FWI2D_VARIANT_SHIFT) & 0xFu;
+    if (forced > (unsigned)kNumStepVariants) return GB_FWI2D_EINVAL;
+    c.variant = forced ? (int)forced - 1 : step_variant_for(d.g, (flags & GB_FWI2D_PLAIN) ? 1 : L.resident);
+    if (!make_call_maps(c, d.g, L, flags)) return GB_FWI2D_ECUDA;
     st = get_tables(d, c.tab);
     if (st) return st;
     if (d.g.pstd) {
@@ -1947,20 +1868,7 @@ static int batch_impl(const gb_fwi2d_params *p, int nsamples, const float *vel, 
     cudaStream_t s = (cudaStream_t)stream;
     long long launches = 0;
     t_enqueue_error = 0;
-    // Kernel variant: forced by the flags, or planned by the tuner (FD mode;
-    // the exact gradient runs the tuned or default variant without trials).
-    const unsigned forced = (flags >> GB_FWI2D_VARIANT_SHIFT) & 0xFu;
-    if (forced > (unsigned)kNumStepVariants) return GB_FWI2D_EINVAL;
-    if (forced) {
-        c.variant = (int)forced - 1;
-    } else if (!d.g.pstd) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess) return GB_FWI2D_ECUDA;
-        const long long wave = (flags & GB_FWI2D_PLAIN) ? 1 : L.resident;
-        const long long ninst = (long long)nsamples * d.g.ns;
-        tune_plan(tune_key(d.g, nsamples, L.resident, flags, dev), exact ? 0 : (ninst + wave - 1) / wave, c);
-    }
-    if ((flags & GB_FWI2D_GRAPH) && !d.g.pstd && c.trials.empty()) {  // transforms and trials run eagerly
+    if ((flags & GB_FWI2D_GRAPH) && !d.g.pstd) {  // transforms run eagerly
         st = run_graph(c, s, launches);
     } else {
         launches = enqueue(c, s);
@@ -2093,13 +2001,7 @@ int gb_fwi2d_tuned_variant(const gb_fwi2d_params *p, int nsamples, int max_resid
     if (st) return st;
     const Layout L = plan_layout(d.g, nsamples, max_resident, true, (flags & GB_FWI2D_FORWARD_ONLY) != 0,
                                  (flags & GB_FWI2D_CHECKPOINT) != 0, (flags & GB_FWI2D_EXACT_GRADIENT) != 0);
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return GB_FWI2D_ECUDA;
-    std::lock_guard<std::mutex> lk(g_tune_mutex);
-    auto it = g_tune.find(tune_key(d.g, nsamples, L.resident, flags, dev));
-    if (it == g_tune.end()) return -1;
-    tune_harvest(it->second);
-    return it->second.done ? it->second.best : -1;
+    return step_variant_for(d.g, (flags & GB_FWI2D_PLAIN) ? 1 : L.resident);
 }
 
 static int static_scratch(void **out);
@@ -2356,8 +2258,8 @@ extern "C" int gb_fwi2d_batch_noalloc(const gb_fwi2d_params *p, int nsamples, co
     c.profile = false;
     c.single_stream = true;  // the two-halves schedule would create a side stream and events
     c.tab.coef = (BlendCoef *)((char *)base + cap);
-    if (!make_maps(c.maps, d.g, (float *)(c.work + L.ring), L.resident)) return GB_FWI2D_ECUDA;
-    if (ckpt && !make_maps(c.maps2, d.g, (float *)(c.work + L.ring2), L.resident)) return GB_FWI2D_ECUDA;
+    c.variant = step_variant_for(d.g, (flags & GB_FWI2D_PLAIN) ? 1 : L.resident);
+    if (!make_call_maps(c, d.g, L, flags)) return GB_FWI2D_ECUDA;
     t_enqueue_error = 0;
     // The weight table is built on the device: no host-to-device copy.
     k_blend_coef<<<1, 32, 0, s>>>(d.g.pml0, c.tab.coef);

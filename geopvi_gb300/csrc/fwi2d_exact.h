@@ -25,7 +25,7 @@
 #if defined(__CUDACC__)
 #define GBX_HD __host__ __device__ __forceinline__
 // Rare paths stay out of line so the hot loops keep a small instruction footprint.
-#define GBX_COLD __host__ __device__ __noinline__
+#define GBX_COLD static __host__ __device__ __noinline__
 #else
 #define GBX_HD inline
 #define GBX_COLD inline
@@ -149,6 +149,59 @@ GBX_HD float round_scaled_to_subnormal(float qs, float rs)
     return gbx_from_bits(sign | n);
 }
 
+// x / y as RN(x*rh + RN(x*rl)), rh = 1/y rounded toward zero and rl = RN(1/y -
+// rh) >= 0: correctly rounded for every x when the host's check of one
+// binade's significands passes for this y (two_op_exact, fwi2d_engine.cu; the
+// method is Brisebarre, Muller & Raina's multiplication by a constant held in
+// two words, 2004) and no term underflows: |x| >= kDivLo, or x = +-0.  rl >= 0
+// keeps the sign of zeros and of infinities.
+GBX_HD float div_two(float x, float rh, float rl) { return gbx_fma(x, rh, gbx_mul(x, rl)); }
+
+// (x / y) / y with both divisions in two operations: valid for x = +-0 and
+// |x| >= kDiv2Lo with y <= 2^20 (the first quotient stays above kDivLo).
+GBX_HD float div2_two(float x, float rh, float rl) { return div_two(div_two(x, rh, rl), rh, rl); }
+
+// rh and rl of div_two for a divisor y in [2^-20, 2^20].
+inline void reciprocal_pair(float y, float *rh, float *rl)
+{
+    const double r = 1.0 / (double)y;
+    float h = (float)r;
+    if ((double)h > r) h = std::nextafter(h, 0.0f);
+    *rh = h;
+    *rl = std::fmax((float)(r - (double)h), 0x1p-149f);  // not 0: an infinite x times rl stays infinite
+}
+
+// Host: every significand of one binade through div_two; a pass holds for
+// every |x| >= kDivLo, since both products and the sum scale with x.
+inline bool two_op_exact(float y)
+{
+    if (!(y >= 0x1p-20f && y <= 0x1p20f)) return false;
+    float rh, rl;
+    reciprocal_pair(y, &rh, &rl);
+    for (uint32_t m = 0; m < (1u << 23); ++m) {
+        const float x = gbx_from_bits(0x3F800000u | m);
+        if (div_two(x, rh, rl) != x / y) return false;
+    }
+    return true;
+}
+
+// Host: the least |x| for which div2_two(x, rh, rl) is (x / y) / y (y passes
+// two_op_exact).  Where x*rl is subnormal its rounding error is up to 2^-150; if
+// no quotient of the binade moves when x*rl is off by 2^-31 of the quotient
+// (true for divisors of few bits, whose quotients keep away from midpoints),
+// that is harmless for quotients down to 2^-118, not only above kDivLo.
+inline float div2_two_least(float y)
+{
+    float rh, rl;
+    reciprocal_pair(y, &rh, &rl);
+    for (uint32_t m = 0; m < (1u << 23); ++m) {
+        const float x = gbx_from_bits(0x3F800000u | m);
+        const float p = gbx_mul(x, rl), e = gbx_mul(gbx_mul(x, rh), 0x1.01p-31f), q = x / y;
+        if (gbx_fma(x, rh, gbx_add(p, e)) != q || gbx_fma(x, rh, gbx_sub(p, e)) != q) return kDiv2Lo;
+    }
+    return std::fmax(0x1p-118f, std::fmin(kDiv2Lo, y * y * 0x1p-117f));
+}
+
 // x / y correctly rounded for every x (y > 0).  On the proved range: the
 // fast path.  Below it (|x| < 2^-100, including subnormals): xs = x * 2^64 is
 // exact and lands inside the range; scaling the quotient back by 2^-64 is
@@ -214,15 +267,38 @@ GBX_HD float div2_any(float x, float y, float r, int fast)
     return div_const2(x, y, r, fast);
 }
 
+GBX_COLD float div2_any_cold(float x, float y, float r, int fast) { return div2_any(x, y, r, fast); }
+
+// xs / y for a scaled dividend xs = x * 2^64 (|x| < kDiv2Lo, two_op_exact(y)),
+// rounded as the float x / y is and scaled alike: q = RN(xs / y) where x / y is
+// normal, |q| >= 2^-62; below that the quotient rounded to the subnormal grid
+// G = 2^-149 * 2^64.  There (|q| + c) - c rounds |q| to even on G, the ulp of
+// [c, 2c); that is the rounding of the true quotient unless q is a midpoint by
+// its own rounding, and then the sign of the remainder decides.
+GBX_HD float div_two_tiny(float xs, float y, float rh, float rl)
+{
+    const float q = div_two(xs, rh, rl), aq = std::fabs(q);
+    const float c = 0x1p-62f, half = 0x1p-86f;
+    float h = gbx_sub(gbx_add(aq, c), c);
+    const float rem = gbx_fma(-aq, y, std::fabs(xs));
+    if (std::fabs(gbx_sub(aq, h)) == half && rem != 0.0f) h = gbx_add(aq, gbx_copysign(half, rem));
+    return aq >= c ? q : gbx_copysign(h, q);
+}
+
+// (x / y) / y for |x| < kDiv2Lo, zeros included.
+GBX_HD float div2_tiny(float x, float y, float rh, float rl)
+{
+    return gbx_mul(div_two_tiny(div_two_tiny(gbx_mul(x, 0x1p64f), y, rh, rl), y, rh, rl), 0x1p-64f);
+}
+
 // Split of 1 - w into floats bh + bl (exact) for the boundary blend, with
 // omw = 1 - w in double.  The host precomputes one per boundary weight and
 // enables the FP32 path only when (1 - w) * q is exact in double for every
 // float q, i.e. 1 - w has at most 29 significant bits.  khi and klo are the
 // bounds of blend_fast's one-FMA path (blend_coef_init).
-struct BlendCoef {
-    float w;
-    float bh, bl;
-    float khi, klo;
+struct alignas(16) BlendCoef {
+    float w, bh, khi2, klo2;  // one 16-byte load: the weight, RN(1 - w), blend_one_fma's bounds
+    float bl, khi, klo;
     double omw;
 };
 
@@ -264,8 +340,12 @@ GBX_HD void blend_coef_init(BlendCoef &c, int i, int pml0)
     c.bl = (float)(c.omw - (double)c.bh);
     c.khi = 0.0f;
     c.klo = 0.0f;
+    c.khi2 = 0.0f;
+    c.klo2 = gbx_from_bits(0x7F800000u);
     if (c.omw == 0.0) {
         c.khi = gbx_from_bits(0x7F800000u);  // +inf
+        c.khi2 = 0x1p127f;
+        c.klo2 = 0.0f;
     } else if (c.bl == 0.0f) {
         const uint64_t b = gbx_dbits(c.omw);
         const int e = (int)((b >> 52) & 0x7FF);  // omw is a normal double in (0, 1]
@@ -282,7 +362,51 @@ GBX_HD void blend_coef_init(BlendCoef &c, int i, int pml0)
         }
         c.khi = gbx_pow2(28 + lam);
         c.klo = gbx_pow2(kb - 28 + lam);
+        c.khi2 = gbx_pow2(27 + lam);
+        c.klo2 = c.klo;
     }
+}
+
+// True when the one-FMA blend fma(bh, q, a) is the reference's value, for any
+// float a and q: blend_coef_init's argument with |a| <= 2^(27+lam) |q| and
+// |a| >= 2^(kb-28+lam) |q|.  Magnitudes near or below 2^-126 only shorten the
+// sum: a's last bit is at 2^-149 or above, so where the products of the test
+// underflow the span of a + bh*q stays far below 53 bits, and the FMA rounds
+// to the subnormal grid as the conversion from double does.  q = 0 passes
+// with a = 0.  Weights with bl != 0 (khi2 = 0, klo2 = inf) never pass, nor do
+// infinities and NaN.
+GBX_HD bool blend_one_fma(float a, float q, float khi2, float klo2)
+{
+    const float aa = std::fabs(a), aq = std::fabs(q);
+    return (aa <= gbx_mul(aq, khi2)) & (aa >= gbx_mul(aq, klo2));
+}
+
+// RN_f(RN_d(a + omw*q)) for any weight with omw = bh + bl, in FP32: true and
+// the value in *out when its rounding is proved.  With u = 2^-24: ph + pl =
+// bh*q and s + e = a + ph exactly; the tail T = e + pl + bl*q is held in t
+// with |t - T| <= u |pl + bl q| + u |t| <= 2^-46 |ph| + 2^-48 |s|, as |pl|,
+// |bl q| <= u |ph|.  r = RN(s + t); |ph| <= 2^11 |r| makes |t| <= 2^-11 |r|, so
+// s - r is exact and d = RN((s - r) + t) is X - r up to 2^-34 |r| / 2 + u |d|
+// for the exact sum X.  The double rounding moves X by at most 2^-53 |X|.
+// r + d (1 + 2^-8) rounding to r says |d| (1 + 2^-8) <= h, h >= 2^-25 |r| the
+// half ulp on that side; for |d| >= h/2 the 2^-8 covers all of those errors
+// ((2^-8 - u) h/2 >= 2^-34 |r|(1 - 2^-16) > 2^-35 |r| + 2^-48 |r| + 2^-52 |r|),
+// and for |d| < h/2 they are far below h/2.  |ph| >= 2^-100 keeps pl exact
+// (q = 0 leaves X = a = s); overflow gives a NaN d, which fails the test.
+GBX_HD bool blend_mix_split(float a, float q, float bh, float bl, float *out)
+{
+    const float ph = gbx_mul(bh, q);
+    const float pl = gbx_fma(bh, q, -ph);
+    const float s = gbx_add(a, ph);
+    const float bv = gbx_sub(s, a);
+    const float e = gbx_add(gbx_sub(a, gbx_sub(s, bv)), gbx_sub(ph, bv));
+    const float t = gbx_add(e, gbx_fma(bl, q, pl));
+    const float r = gbx_add(s, t);
+    const float d = gbx_add(gbx_sub(s, r), t);
+    const float aph = std::fabs(ph);
+    *out = q == 0.0f ? s : r;  // s = a + (+-0): the sign of a zero sum as in double
+    return (gbx_fma(d, 0x1.01p0f, r) == r) & (aph <= gbx_mul(std::fabs(r), 2048.0f)) &
+           ((aph >= 0x1p-100f) | (q == 0.0f));
 }
 
 // RN_f(RN_d(a + omw * q)) for a = RN_f(w * ext), computed in FP32.

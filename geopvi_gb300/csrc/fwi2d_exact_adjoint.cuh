@@ -25,6 +25,10 @@
 
 namespace gbfwi {
 
+constexpr int kTileZ = 16;  // rows per tile of the adjoint kernel
+constexpr int kHaloX = 8;   // halo columns of its staged tiles (TMA x offsets stay 16-byte aligned)
+constexpr int kBoxX = kTileX + 2 * kHaloX;
+
 struct ExactBatch {
     const float *vdt;      // [nsamples][fstride] padded v*dt
     const float *abeta;    // [nsamples][fstride] (v dt)^2 beta on stencil cells, 0 elsewhere
@@ -175,7 +179,7 @@ constexpr int kAdjMinBlocks = 5;  // resident blocks per SM: each waits on its t
 
 template <int H>
 struct AdjShape {
-    static constexpr int kTile = TileShape<H>::kP1Floats;  // floats of one staged tile
+    static constexpr int kTile = (kTileZ + 2 * H) * kBoxX;  // floats of one staged tile
     static constexpr int kBytes = 2 * 4 * kTile;            // TMA bytes per block
     static constexpr int kSmem = kBytes + 16;               // + the mbarrier
 };
@@ -193,7 +197,8 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
     const int slot = blockIdx.y;
     const int inst = b.inst0 + slot;
     const int sample = inst / g.ns, shot = inst - sample * g.ns;
-    const int trow = blockIdx.x / g.tiles_x, tcol = blockIdx.x - trow * g.tiles_x;
+    const int tiles_x = g.pitch / kTileX;
+    const int trow = blockIdx.x / tiles_x, tcol = blockIdx.x - trow * tiles_x;
     const int col0 = tcol * kTileX, row0 = trow * kTileZ;
     const int lane = threadIdx.x & 31, rr0 = threadIdx.x >> 5;  // tile rows rr0 + q * RS
     if (threadIdx.x == 0) {

@@ -63,7 +63,7 @@ class Fwi2dEngine:
         self.graph = graph
         self.plain = plain
         self.checkpoint = checkpoint
-        self.variant = variant  # FD step kernel variant; None: the library's tuner picks
+        self.variant = variant  # FD step kernel variant; None: the library picks by the work of a launch
         self._cp = params.c()
         self._work: torch.Tensor | None = None
         self._work_key = None
@@ -182,8 +182,8 @@ class Fwi2dEngine:
 
     def tuned_variant(self, nsamples: int, *, imaging: bool = False, forward_only: bool = False,
                       exact: bool = False) -> int:
-        """The FD step variant the tuner settled on for batches of ``nsamples``
-        run with the given mode (-1 while variants remain untried)."""
+        """The FD step variant the library runs for batches of ``nsamples`` in
+        the given mode."""
         flags = (_native.FLAG_IMAGING if imaging else 0) | (_native.FLAG_PLAIN if self.plain else 0) | \
             (_native.FLAG_CHECKPOINT if self.checkpoint else 0) | \
             (_native.FLAG_FORWARD_ONLY if forward_only else 0) | (_native.FLAG_EXACT_GRADIENT if exact else 0)
