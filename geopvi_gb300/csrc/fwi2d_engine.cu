@@ -573,43 +573,6 @@ static int get_tables(const Derived &d, DeviceTables &out)
 // Launch sequence
 // ---------------------------------------------------------------------------
 
-// cuTensorMapEncodeTiled, fetched from the driver through the runtime.
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
-{
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
-    });
-    return fn;
-}
-
-// Encoding a tensor map needs a current driver context, and a host thread
-// that has made no runtime call that binds one (cudaGetDevice and
-// cudaGetLastError do not) has none.  Bind the current device's primary
-// context then -- but leave a context the caller made current alone.
-static bool ensure_context()
-{
-    static PFN_cuCtxGetCurrent_v4000 get_current = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 4000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<PFN_cuCtxGetCurrent_v4000>(f);
-    });
-    CUcontext ctx = nullptr;
-    if (get_current && get_current(&ctx) == CUDA_SUCCESS && ctx) return true;
-    int dev = 0;
-    return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
-}
-
 // A 3-D fp32 tensor map over `depth` padded fields [depth][ntz][pitch] with a
 // (box_x, box_z, 1) box; out-of-range elements of a box read as zero.
 static bool make_map(CUtensorMap &m, void *base, const Geom &g, long long depth, int box_x, int box_z)

@@ -25,6 +25,7 @@
 
 #include "fd_weights.cuh"
 #include "fwi2d_exact.h"
+#include "tma.cuh"
 
 namespace gbfwi {
 
@@ -175,69 +176,6 @@ __device__ __forceinline__ float padded_velocity(const Geom &g, const float *vel
     int jz = min(max(iz - g.pml, 0), g.nz - 1);
     int jx = min(max(ix - g.pml, 0), g.nx - 1);
     return vel[(long long)jz * g.nx + jx];
-}
-
-// ---------------------------------------------------------------------------
-// TMA / mbarrier helpers (inline PTX)
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void *p)
-{
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void fence_barrier_init()
-{
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// 3-D tiled TMA load into shared memory, completing on `bar`.
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y,
-                                            int z)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Bounded wait: true once phase `parity` completed, false after the limit
-// (the caller records the timeout and skips its work).
-// Programmatic dependent launch: wait for the previous grid on the stream
-// (complete, its writes visible), and let the next one be scheduled.  Both
-// are no-ops in a launch without the programmatic-serialization attribute.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity)
-{
-    for (int i = 0; i < (1 << 24); ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
 }
 
 }  // namespace gbfwi

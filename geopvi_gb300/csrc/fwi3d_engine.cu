@@ -6,18 +6,34 @@
 // same FP32 operations, and this engine reproduces them bit for bit.
 //
 // Per time step of a wave of resident (sample, shot) solves:
-//   k3_step    stencil + the six absorbing passes for every padded cell, and
-//              the stored d2p/dt2 (forward) or the imaging term (adjoint) of
-//              the interior cells;
-//   k3_io_fwd  source injection (and the stored value at the source cell),
-//              then receiver sampling;  k3_io_adj  residual injection at the
-//              receivers (and their imaging terms).
-// k3_step: one thread per (x, y) column of a 32 x 8 tile, marching along z
-// through a chunk of planes with the z stencil window in registers; x and y
-// neighbours come through the read-only cache.  Fields are [z][y][x] with a
-// row pitch of 32 floats.  The adjoint runs the same operator backwards; its
-// forward field is stored whole or, with GB_FWI3D_CHECKPOINT, as
-// ceil(sqrt(nt))-step segments recomputed from checkpoints.
+//   k3_step    stencil + the six absorbing passes for every updated cell, source
+//              injection, and the stored d2p/dt2 (forward) or the imaging term
+//              (adjoint) of the interior cells; blocks of its own sample the
+//              receivers of the step before;
+//   k3_io_adj  adjoint only: residual injection at the receivers (and their
+//              imaging terms).
+// k3_step: a block owns 64 x 16 columns -- eight warps, each lane two columns of
+// two rows -- and marches along z through a chunk of planes.  These arrive by
+// TMA in a ring of shared-memory stages, several planes ahead (mbarriers both
+// ways; the warps take turns at issuing): p1 with its x and y halo, and p0 and
+// v*dt.  The z windows slide in registers.  The z and y passes are uniform over
+// a warp's row; the x pass, which few of a row's cells need, is done afterwards
+// by as many lanes as there are strip cells, packed.  The rim (cells outside [L, n - L)), which the
+// scheme never changes from zero, is not visited: the ring is cleared once.
+// Fields are [z][y][x], the first updated column on a 32-byte boundary.  The
+// adjoint runs the same operator backwards; its forward field is stored whole
+// or, with GB_FWI3D_CHECKPOINT, as ceil(sqrt(nt))-step segments recomputed from
+// checkpoints.
+//
+// What bounds it: instructions (470 / 565 per warp and plane of 128 cells,
+// forward / adjoint, of which 124 are the stencil's; schedulers issue on 60 % of
+// their cycles with 16 warps an SM), DRAM at 2.2 TB/s.  Measured on 160^3 cells, 4
+// shots, 200 steps of misfit + gradient: 104 ms with one column a thread reading
+// its 16 x and y taps from global memory (219 instructions per 32 cells), 87 ms
+// with the planes of p1 staged (two columns a lane, 8 rows), 93 ms with two rows a
+// lane and the x pass in place, 79 ms with the x pass packed, 73 ms with tiles of
+// interior columns compiled apart.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,28 +44,14 @@
 #include "../../include/geopvi_fwi2d.h"
 #include "../../include/geopvi_fwi3d.h"
 #include "fd_weights.cuh"
+#include "tma.cuh"
 
 namespace gbfwi3 {
 
-using gbfwi::fd_weight;
+using namespace gbfwi;
 
-// Build-time tuning knobs: planes per z chunk (each chunk reloads 2H planes
-// of the z window) and resident blocks per SM the registers are capped for.
-#ifndef GB_FWI3D_ZCHUNK
-#define GB_FWI3D_ZCHUNK 32
-#endif
-#ifndef GB_FWI3D_MIN_BLOCKS
-#define GB_FWI3D_MIN_BLOCKS 4
-#endif
-#ifndef GB_FWI3D_ZUNROLL
-#define GB_FWI3D_ZUNROLL 1
-#endif
-#define GB_FWI3D_PRAGMA(x) _Pragma(#x)
-#define GB_FWI3D_UNROLL(n) GB_FWI3D_PRAGMA(unroll n)
-
-constexpr int kBX = 32;     // tile columns (x), one warp
-constexpr int kBY = 8;      // tile rows (y)
-constexpr int kZC = GB_FWI3D_ZCHUNK;  // planes per z chunk
+constexpr int kBX = 64;          // tile columns (x): one warp, two a lane
+constexpr int kBlocksPerSM = 2;  // 128 registers a thread
 constexpr int kMisfitBlocks = 64;
 
 struct Geom3 {
@@ -57,10 +59,12 @@ struct Geom3 {
     int nx, ny, nz;
     int L, pml, pml0;
     int nt, nti, ns, nr, nu;   // nu: distinct receiver cells
-    int tiles_x, tiles_y, chunks_z;
+    int xoff, ioff, ipitch;    // memory column of x = 0, of interior x = 0, and the interior row pitch
+    int tiles_x, tiles_y;
     long long sz;              // z stride (pitch * nty)
     long long fstride;         // floats per padded field
-    long long istride;         // floats per interior field (nx * ny * nz)
+    long long istride;         // floats per interior field (ipitch * ny * nz)
+    long long ncell;           // model cells
     float id[3], id2[3];       // 1/d and 1/d^2 for x, y, z
     float idt2, dt;
 };
@@ -80,6 +84,46 @@ struct Batch3 {
     const int *uidx;            // [nr]
     int nsnap;                  // stored steps per resident solve
     int inst0;                  // first solve of the wave
+    int *status;                // nonzero: a bounded wait gave up, results are set to NaN
+};
+
+// One step: ring buffers (k, k+1, k+2) mod 3 = p0, p1, p2.
+struct Step3 {
+    int k;
+    int snap;    // >= 0: the slot's stored-field index written (forward) or read (adjoint)
+    float wav;   // source value (forward)
+    int chunks, planes;   // z chunks and planes per chunk
+    int sample_it;        // >= 0: sampling blocks record p1 as the data of this time index
+    int sample_blocks;    // ... blocks per solve, after the tiles'
+};
+
+// Shape of a tile and what k3_step stages of it: kStages planes of p1 with their
+// halo, and kPairs planes of p0 and v*dt.  A plane's p0 and v*dt travel with the
+// p1 plane H ahead of it, under the same barrier.
+template <int H>
+struct Stage3 {
+    static constexpr int kWarps = H <= 5 ? 8 : 6;  // two blocks' stages fit an SM
+    static constexpr int kBY = 2 * kWarps;         // tile rows (y): two a warp
+    static constexpr int kHaloX = H <= 4 ? 4 : 8;
+    static constexpr int kX = kBX + 2 * kHaloX, kY = kBY + 2 * H;
+    static constexpr int kBytes = 4 * kX * kY;
+    static constexpr int kPitch = (kBytes + 127) / 128 * 32;  // floats from stage to stage
+    static constexpr int kStages = H <= 4 ? H + 5 : 9;
+    // A stage is free when the tap plane in it is done with; then so are p0 and
+    // v*dt of that plane, kStages - H planes before those that go with the refill.
+    static constexpr int kPairs = kStages - H;
+    static constexpr int kOwn = kBX * kBY;  // the tile's own cells of a plane
+    static constexpr int kPairBase = kStages * kPitch;
+    static constexpr int kScratch = kPairBase + kPairs * 2 * kOwn;  // each warp's new values, for the x pass
+    static constexpr int kBarriers = kScratch + kWarps * 2 * kBX;
+    static constexpr int kSmem = 4 * kBarriers + 16 * kStages;
+    static constexpr int kThreads = 32 * kWarps;
+};
+
+// Tensor maps: p1's planes with halo and the tile's own cells over a ring, and
+// the own cells over v*dt.
+struct Maps3 {
+    CUtensorMap p1, p0, vdt;
 };
 
 __device__ __forceinline__ float fmaf_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
@@ -113,146 +157,14 @@ __device__ __forceinline__ float blend(float q, float s, float w, float omw, flo
     return fmaf_rn(w, e, __fmul_rn(omw, q));
 }
 
-// One time step of every resident solve.  blockIdx.x = tile (x fastest, then
-// y, then z chunk), blockIdx.y = resident slot.  k: step within the pass
-// (ring buffers (k, k+1, k+2) mod 3 = p0, p1, p2); snap >= 0: the slot's
-// stored-field index written (forward) or read (adjoint) at this step.
-template <int H, bool ADJ>
-__global__ void __launch_bounds__(kBX *kBY, GB_FWI3D_MIN_BLOCKS) k3_step(const Geom3 g, const Batch3 b, int k, int snap)
-{
-    const int slot = blockIdx.y;
-    int t = blockIdx.x;
-    const int tx = t % g.tiles_x;
-    t /= g.tiles_x;
-    const int ty = t % g.tiles_y;
-    const int cz = t / g.tiles_y;
-    const int x = tx * kBX + threadIdx.x, y = ty * kBY + threadIdx.y;
-    if (x >= g.ntx || y >= g.nty) return;
-    const int z0 = cz * kZC, z1 = min(z0 + kZC, g.ntz);
-    const int inst = b.inst0 + slot;
-    const int sample = inst / g.ns;
-    float *ring = b.ring + (long long)slot * 3 * g.fstride;
-    const float *__restrict__ p0 = ring + (long long)(k % 3) * g.fstride;
-    const float *__restrict__ p1 = ring + (long long)((k + 1) % 3) * g.fstride;
-    float *__restrict__ p2 = ring + (long long)((k + 2) % 3) * g.fstride;
-    const long long col = (long long)y * g.pitch + x;
-    const int L = g.L;
-    if (x < L || x >= g.ntx - L || y < L || y >= g.nty - L) {  // rim column: always zero
-        for (int z = z0; z < z1; ++z) p2[z * g.sz + col] = 0.0f;
-        return;
-    }
-    const float *vdc = b.vdt + (long long)sample * g.fstride + col;
-    const bool xmin = x < g.pml, xmax = x >= g.ntx - g.pml;
-    const bool ymin = y < g.pml, ymax = y >= g.nty - g.pml;
-    const bool inner_xy = !(xmin || xmax || ymin || ymax);
-    float *sv = nullptr, *Gv = nullptr;
-    if (snap >= 0 && inner_xy) {
-        const long long j0 = (long long)(y - g.pml) * g.nx + (x - g.pml);
-        sv = b.snap + ((long long)slot * b.nsnap + snap) * g.istride + j0;
-        if (ADJ) Gv = b.G + (long long)inst * g.istride + j0;
-    }
-    const long long ps = (long long)g.nx * g.ny;  // interior plane stride
-    const long long sy = g.pitch;
-
-    float win[2 * H + 1];
-#pragma unroll
-    for (int m = 0; m < 2 * H; ++m) {
-        const int zz = z0 - H + m;
-        win[m] = (zz >= 0 && zz < g.ntz) ? __ldg(p1 + zz * g.sz + col) : 0.0f;
-    }
-    // this plane's window value, p0 and v*dt, loaded one plane ahead
-    float wn = z0 + H < g.ntz ? __ldg(p1 + (z0 + H) * g.sz + col) : 0.0f;
-    float p0n = __ldg(p0 + z0 * g.sz + col), vdn = __ldg(vdc + z0 * g.sz);
-    // adjoint stored step: the stored field and the accumulator, also a plane ahead
-    float svn = 0.0f, gvn = 0.0f;
-    if (ADJ && sv && z0 >= g.pml && z0 < g.ntz - g.pml) {
-        const long long j = (long long)(z0 - g.pml) * ps;
-        svn = __ldg(sv + j);
-        gvn = Gv[j];
-    }
-    GB_FWI3D_UNROLL(GB_FWI3D_ZUNROLL)
-    for (int z = z0; z < z1; ++z) {
-        win[2 * H] = wn;
-        const float p0c = p0n, vd = vdn;
-        const float svc = svn, gvc = gvn;
-        if (z + 1 < z1) {
-            const int zn = z + 1 + H;
-            wn = zn < g.ntz ? __ldg(p1 + zn * g.sz + col) : 0.0f;
-            p0n = __ldg(p0 + (z + 1) * g.sz + col);
-            vdn = __ldg(vdc + (z + 1) * g.sz);
-            if (ADJ && sv && z + 1 >= g.pml && z + 1 < g.ntz - g.pml) {
-                const long long j = (long long)(z + 1 - g.pml) * ps;
-                svn = __ldg(sv + j);
-                gvn = Gv[j];
-            }
-        }
-        const long long c = z * g.sz + col;
-        float q = 0.0f;
-        if (z >= L && z < g.ntz - L) {
-            const float pc = win[H];
-            float lx = __fmul_rn(fd_weight<H>(0), pc), ly = lx, lz = lx;
-#pragma unroll
-            for (int m = 1; m <= H; ++m) {
-                lx = fmaf_rn(fd_weight<H>(m), __fadd_rn(__ldg(p1 + c + m), __ldg(p1 + c - m)), lx);
-                ly = fmaf_rn(fd_weight<H>(m), __fadd_rn(__ldg(p1 + c + m * sy), __ldg(p1 + c - m * sy)), ly);
-                lz = fmaf_rn(fd_weight<H>(m), __fadd_rn(win[H + m], win[H - m]), lz);
-            }
-            float tt = __fmul_rn(lz, g.id2[2]);
-            tt = fmaf_rn(ly, g.id2[1], tt);
-            tt = fmaf_rn(lx, g.id2[0], tt);
-            const float u = fmaf_rn(2.0f, pc, -p0c);
-            q = fmaf_rn(__fmul_rn(vd, vd), tt, u);
-            const bool zmin = z < g.pml, zmax = z >= g.ntz - g.pml;
-            if (zmin) {
-                const int wi = z - L;
-                const long long d = g.sz;
-                q = blend(q, __fmul_rn(vd, g.id[2]), b.w[wi], b.omw[wi], pc, win[H + 1], win[H + 2], p0c,
-                          __ldg(p0 + c + d), __ldg(p0 + c + 2 * d), __ldg(p0 + c + 3 * d), __ldg(p0 + c + 4 * d));
-            }
-            if (zmax) {
-                const int wi = g.ntz - L - 1 - z;
-                const long long d = -g.sz;
-                q = blend(q, __fmul_rn(vd, g.id[2]), b.w[wi], b.omw[wi], pc, win[H - 1], win[H - 2], p0c,
-                          __ldg(p0 + c + d), __ldg(p0 + c + 2 * d), __ldg(p0 + c + 3 * d), __ldg(p0 + c + 4 * d));
-            }
-            if (!inner_xy) {
-                if (ymin || ymax) {
-                    const int wi = ymin ? y - L : g.nty - L - 1 - y;
-                    const long long d = ymin ? sy : -sy;
-                    q = blend(q, __fmul_rn(vd, g.id[1]), b.w[wi], b.omw[wi], pc, __ldg(p1 + c + d),
-                              __ldg(p1 + c + 2 * d), p0c, __ldg(p0 + c + d), __ldg(p0 + c + 2 * d),
-                              __ldg(p0 + c + 3 * d), __ldg(p0 + c + 4 * d));
-                }
-                if (xmin || xmax) {
-                    const int wi = xmin ? x - L : g.ntx - L - 1 - x;
-                    const long long d = xmin ? 1 : -1;
-                    q = blend(q, __fmul_rn(vd, g.id[0]), b.w[wi], b.omw[wi], pc, __ldg(p1 + c + d),
-                              __ldg(p1 + c + 2 * d), p0c, __ldg(p0 + c + d), __ldg(p0 + c + 2 * d),
-                              __ldg(p0 + c + 3 * d), __ldg(p0 + c + 4 * d));
-                }
-            }
-            if (sv && z >= g.pml && z < g.ntz - g.pml) {
-                const long long j = (long long)(z - g.pml) * ps;
-                if (!ADJ)
-                    sv[j] = __fmul_rn(__fsub_rn(q, u), g.idt2);
-                else
-                    Gv[j] = fmaf_rn(svc, q, gvc);
-            }
-        }
-        p2[c] = q;
-#pragma unroll
-        for (int m = 0; m < 2 * H; ++m) win[m] = win[m + 1];
-    }
-}
-
 __device__ __forceinline__ long long padded_cell(const Geom3 &g, const int *xyz)
 {
-    return (long long)(xyz[2] + g.pml) * g.sz + (long long)(xyz[1] + g.pml) * g.pitch + (xyz[0] + g.pml);
+    return (long long)(xyz[2] + g.pml) * g.sz + (long long)(xyz[1] + g.pml) * g.pitch + (xyz[0] + g.pml + g.xoff);
 }
 
 __device__ __forceinline__ long long interior_cell(const Geom3 &g, const int *xyz)
 {
-    return ((long long)xyz[2] * g.ny + xyz[1]) * g.nx + xyz[0];
+    return ((long long)xyz[2] * g.ny + xyz[1]) * g.ipitch + xyz[0] + g.ioff;
 }
 
 __device__ __forceinline__ float model_velocity(const Geom3 &g, const float *vel, const int *xyz)
@@ -260,33 +172,351 @@ __device__ __forceinline__ float model_velocity(const Geom3 &g, const float *vel
     return vel[((long long)xyz[1] * g.nx + xyz[0]) * g.nz + xyz[2]];
 }
 
-// Forward IO of step k (time it): source injection at the shot's cell (and
-// the stored d2p/dt2 there, which must include it), then the receivers.
-__global__ void k3_io_fwd(const Geom3 g, const Batch3 b, int k, int it, float wav, int snap, int record)
+// The cell's new level from its taps (x[m], y[m], z[m]: m cells away) before
+// the absorbing passes; u = 2 p1 - p0.
+template <int H>
+__device__ __forceinline__ float update3(const Geom3 &g, const float *x, const float *y, const float *z, float p0c,
+                                         float vd, float *u)
 {
-    const int slot = blockIdx.x;
+    const float pc = z[0];
+    float lx = __fmul_rn(fd_weight<H>(0), pc), ly = lx, lz = lx;
+#pragma unroll
+    for (int m = 1; m <= H; ++m) {
+        lx = fmaf_rn(fd_weight<H>(m), __fadd_rn(x[m], x[-m]), lx);
+        ly = fmaf_rn(fd_weight<H>(m), __fadd_rn(y[m], y[-m]), ly);
+        lz = fmaf_rn(fd_weight<H>(m), __fadd_rn(z[m], z[-m]), lz);
+    }
+    float t = __fmul_rn(lz, g.id2[2]);
+    t = fmaf_rn(ly, g.id2[1], t);
+    t = fmaf_rn(lx, g.id2[0], t);
+    *u = fmaf_rn(2.0f, pc, -p0c);
+    return fmaf_rn(__fmul_rn(vd, vd), t, *u);
+}
+
+// One face's blend of a cell along an axis: p0 points at the cell, d leads one
+// cell inward, x1 and x2 are p1 at 1 and 2 cells inward, wi the weight index.
+__device__ __forceinline__ float face(const Batch3 &b, float q, float s, int wi, float pc, float x1, float x2,
+                                      const float *p0, float p0c, long long d)
+{
+    return blend(q, s, __ldg(b.w + wi), __ldg(b.omw + wi), pc, x1, x2, p0c, __ldg(p0 + d), __ldg(p0 + 2 * d),
+                 __ldg(p0 + 3 * d), __ldg(p0 + 4 * d));
+}
+
+// Receivers of one resident solve: p1 (the level of time index it) into syn.
+__device__ __forceinline__ void sample3(const Geom3 &g, const Batch3 &b, const float *p, int inst, int it, int first,
+                                        int stride)
+{
+    float *out = b.syn + ((long long)inst * g.nt + it) * g.nr;
+    for (int r = first; r < g.nr; r += stride) out[r] = __ldg(p + padded_cell(g, b.rec + 3 * r));
+}
+
+__device__ __forceinline__ float2 shared2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
+
+// Two columns' store, whole or (EDGE) what is valid of it; STREAM: written once,
+// read much later.
+template <bool EDGE, bool STREAM>
+__device__ __forceinline__ void store2(float *p, float u, float v, bool a, bool b)
+{
+    if (!EDGE) {
+        const float2 t = make_float2(u, v);
+        if (STREAM) __stcs(reinterpret_cast<float2 *>(p), t);
+        else *reinterpret_cast<float2 *>(p) = t;
+        return;
+    }
+    if (a) p[0] = u;
+    if (b) p[1] = v;
+}
+
+// A tile of one step: planes z0..z1-1 of the rows and columns from y0, x0 on.
+// Without EDGE its columns are all interior.
+template <int H, bool ADJ, bool EDGE>
+__device__ __forceinline__ void march3(const Maps3 &tm, const Geom3 &g, const Batch3 &b, const Step3 &sa, float *smem,
+                                       int x0, int y0, int z0, int z1)
+{
+    using ST = Stage3<H>;
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + ST::kBarriers), *empty = full + ST::kStages;
+    const int slot = blockIdx.y;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int inst = b.inst0 + slot;
     const int sample = inst / g.ns, shot = inst - sample * g.ns;
     float *ring = b.ring + (long long)slot * 3 * g.fstride;
-    const float *p0 = ring + (long long)(k % 3) * g.fstride;
-    const float *p1 = ring + (long long)((k + 1) % 3) * g.fstride;
-    float *p2 = ring + (long long)((k + 2) % 3) * g.fstride;
+    const int L = g.L;
     if (threadIdx.x == 0) {
-        const int *s = b.src + 3 * shot;
-        const long long c = padded_cell(g, s);
-        const float v = model_velocity(g, b.vel + (long long)sample * g.istride, s);
-        const float q = __fadd_rn(p2[c], inject(wav, g.dt, v));
-        p2[c] = q;
-        if (snap >= 0) {
-            const float u = fmaf_rn(2.0f, p1[c], -p0[c]);
-            b.snap[((long long)slot * b.nsnap + snap) * g.istride + interior_cell(g, s)] =
-                __fmul_rn(__fsub_rn(q, u), g.idt2);
+        for (int i = 0; i < ST::kStages; ++i) {
+            mbar_init(full + i, 1);
+            mbar_init(empty + i, ST::kWarps);
+        }
+        fence_barrier_init();
+    }
+    __syncthreads();
+
+    // This lane's columns x, x + 1 of the rows y, y + 1.
+    const int x = x0 + 2 * lane, y = y0 + 2 * warp;
+    const bool ia = !EDGE || (x >= g.pml && x < g.ntx - g.pml);
+    const bool ib = !EDGE || (x + 1 >= g.pml && x + 1 < g.ntx - g.pml);
+    // Columns of the tile in the left and in the right strip: [L, pml) and
+    // [ntx - pml, ntx - L) cut to it.
+    const int xe = min(x0 + kBX, g.ntx - L), lx1 = min(xe, g.pml), rx0 = max(x0, g.ntx - g.pml);
+    const int nl = max(0, lx1 - x0), nx = nl + max(0, xe - rx0);
+    float *scratch = smem + ST::kScratch + warp * 2 * kBX;
+    bool row[2], yin[2];  // updated, interior
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        row[r] = y + r < g.nty - L;
+        yin[r] = row[r] && y + r >= g.pml && y + r < g.nty - g.pml;
+    }
+    const bool yl = y < g.nty / 2;
+    const int *src = b.src + 3 * shot;
+    const int sy = ADJ ? -1 : __ldg(src + 1) + g.pml;
+    const int sz = ADJ || (y != sy && y + 1 != sy) ? -1 : __ldg(src + 2) + g.pml;  // the source's plane, if in these rows
+
+    // Everything above reads only what is constant through the call; the
+    // previous step must be complete below.
+    grid_dependency_wait();
+    grid_launch_dependents();
+    bool ok = true;  // no wait has given up
+    // Plane i of the chunk, z0 - H + i, into its stage once every warp has
+    // released the one before.
+    const int nplanes = z1 - z0 + 2 * H;
+    auto issue = [&](int i) {
+        const int st = i % ST::kStages, use = i / ST::kStages;
+        if (use > 0) ok = ok && mbar_wait_bounded(empty + st, (use - 1) & 1);
+        if (!ok) return;
+        mbar_arrive_expect_tx(full + st, ST::kBytes + (i >= 2 * H ? 8 * ST::kOwn : 0));
+        tma_load_4d(smem + st * ST::kPitch, &tm.p1, full + st, x0 + g.xoff - ST::kHaloX, y0 - H, z0 - H + i,
+                    slot * 3 + (sa.k + 1) % 3);
+        if (i >= 2 * H) {  // the last p1 plane of plane z0 + i - 2H, which goes with it
+            const int n = i - 2 * H;
+            float *pair = smem + ST::kPairBase + n % ST::kPairs * 2 * ST::kOwn;
+            tma_load_4d(pair, &tm.p0, full + st, x0 + g.xoff, y0, z0 + n, slot * 3 + sa.k % 3);
+            tma_load_4d(pair + ST::kOwn, &tm.vdt, full + st, x0 + g.xoff, y0, z0 + n, sample);
+        }
+    };
+    if (threadIdx.x == 0)
+        for (int i = 0; i < min(ST::kStages, nplanes); ++i) issue(i);
+
+    const long long col = z0 * g.sz + (long long)y * g.pitch + x + g.xoff;
+    float *p2 = ring + (long long)((sa.k + 2) % 3) * g.fstride + col;
+    const float *p0 = ring + (long long)(sa.k % 3) * g.fstride + col;
+    const long long ps = (long long)g.ipitch * g.ny;  // interior plane stride
+    float *sv = nullptr, *Gv = nullptr;
+    if (sa.snap >= 0) {
+        const long long j0 = ((long long)(z0 - g.pml) * g.ny + (y - g.pml)) * g.ipitch + (x - g.pml + g.ioff);
+        sv = b.snap + ((long long)slot * b.nsnap + sa.snap) * g.istride + j0;
+        if (ADJ) Gv = b.G + (long long)inst * g.istride + j0;
+    }
+    const int mine = (2 * warp + H) * ST::kX + ST::kHaloX + 2 * lane;  // this lane's place in a staged plane
+
+    // The z windows: wa, wb[r][H + m] = plane z + m of row r's two columns.  The
+    // chunk's first 2H planes only fill them; the first H of those are then free.
+    float wa[2][2 * H + 1], wb[2][2 * H + 1];
+#pragma unroll
+    for (int i = 0; i < 2 * H; ++i) {
+        // planes beyond the first kStages: one for every stage freed two steps ago
+        if (i >= 2 && i < H + 2 && threadIdx.x == 0 && i - 2 + ST::kStages < nplanes) issue(i - 2 + ST::kStages);
+        ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(full + i % ST::kStages, (i / ST::kStages) & 1));
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float2 v = shared2(smem + i % ST::kStages * ST::kPitch + mine + r * ST::kX);
+            wa[r][i] = v.x;
+            wb[r][i] = v.y;
+        }
+        if (i < H) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + i % ST::kStages);
         }
     }
-    if (!record) return;
-    __syncthreads();
-    float *out = b.syn + ((long long)inst * g.nt + it) * g.nr;
-    for (int r = threadIdx.x; r < g.nr; r += blockDim.x) out[r] = p2[padded_cell(g, b.rec + 3 * r)];
+    // Issued so far: kStages, and one for each i above.
+    constexpr int kAhead = ST::kStages + (2 * H < H + 2 ? 2 * H : H + 2) - 2;
+    int tap = H % ST::kStages, front = 2 * H % ST::kStages;  // stages of plane z and of plane z + H
+    int front_phase = (2 * H / ST::kStages) & 1;
+    int pair0 = ST::kPairBase;                               // p0 and v*dt of plane z
+    // Adjoint stored step: the stored field and the accumulator, one plane ahead.
+    float2 svn[2], gvn[2];
+    auto load_terms = [&](int z, const float *s, const float *G) {
+        if (ADJ && sv && (ia || ib) && z >= g.pml && z < g.ntz - g.pml) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+                if (yin[r]) {
+                    svn[r] = __ldcs(reinterpret_cast<const float2 *>(s + r * g.ipitch));
+                    gvn[r] = *reinterpret_cast<const float2 *>(G + r * g.ipitch);
+                }
+        }
+    };
+    load_terms(z0, sv, Gv);
+#pragma unroll 1
+    for (int z = z0; z < z1 && ok; ++z) {
+        // One more plane, into the stage that every warp released two planes ago.
+        const int next = z - z0 + H - 2 + ST::kStages;
+        if (lane == 0 && warp == (z - z0) % ST::kWarps && next >= kAhead && next < nplanes) issue(next);
+        const bool zin = z >= g.pml && z < g.ntz - g.pml;
+        const bool stored = sv && zin;
+        float2 svc[2], gvc[2];
+        if (ADJ) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                svc[r] = svn[r];
+                gvc[r] = gvn[r];
+            }
+            if (z + 1 < z1) load_terms(z + 1, sv + ps, Gv + ps);
+        }
+        ok = ok && mbar_wait_bounded(full + front, front_phase);
+        const float *pl = smem + tap * ST::kPitch + mine, *pf = smem + front * ST::kPitch + mine;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float2 v = shared2(pf + r * ST::kX);
+            wa[r][2 * H] = v.x;
+            wb[r][2 * H] = v.y;
+        }
+        // The columns' y neighbours: rows -H .. H + 1, the lane's own two at H, H + 1.
+        float ya[2 * H + 2], yb[2 * H + 2];
+#pragma unroll
+        for (int m = 0; m < 2 * H + 2; ++m) {
+            if (m == H || m == H + 1) {
+                ya[m] = wa[m - H][H];
+                yb[m] = wb[m - H][H];
+                continue;
+            }
+            const float2 v = shared2(pl + (m - H) * ST::kX);
+            ya[m] = v.x;
+            yb[m] = v.y;
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            constexpr int K = (H + 1) / 2;  // pairs on each side that hold the x taps
+            float xt[4 * K + 2];
+#pragma unroll
+            for (int k = -K; k <= K; ++k) {
+                if (k == 0) continue;
+                const float2 v = shared2(pl + r * ST::kX + 2 * k);
+                xt[2 * (K + k)] = v.x;
+                xt[2 * (K + k) + 1] = v.y;
+            }
+            xt[2 * K] = wa[r][H];
+            xt[2 * K + 1] = wb[r][H];
+            const float *own = smem + pair0 + (2 * warp + r) * kBX + 2 * lane;
+            const float2 p0c = shared2(own), vd = shared2(own + ST::kOwn);
+            float ua, ub;
+            float qa = update3<H>(g, xt + 2 * K, ya + H + r, wa[r] + H, p0c.x, vd.x, &ua);
+            float qb = update3<H>(g, xt + 2 * K + 1, yb + H + r, wb[r] + H, p0c.y, vd.y, &ub);
+            if (row[r]) {
+                // The absorbing passes: z, then y, then x (at most one face each)
+                const float *p0r = p0 + r * g.pitch;
+                if (!zin) {
+                    const bool zl = z < g.pml;
+                    const int wi = zl ? z - L : g.ntz - L - 1 - z;
+                    const long long d = zl ? g.sz : -g.sz;
+                    qa = face(b, qa, __fmul_rn(vd.x, g.id[2]), wi, wa[r][H], zl ? wa[r][H + 1] : wa[r][H - 1],
+                              zl ? wa[r][H + 2] : wa[r][H - 2], p0r, p0c.x, d);
+                    qb = face(b, qb, __fmul_rn(vd.y, g.id[2]), wi, wb[r][H], zl ? wb[r][H + 1] : wb[r][H - 1],
+                              zl ? wb[r][H + 2] : wb[r][H - 2], p0r + 1, p0c.y, d);
+                }
+                if (!yin[r]) {
+                    const int wi = yl ? y + r - L : g.nty - L - 1 - y - r;
+                    const long long d = yl ? g.pitch : -g.pitch;
+                    qa = face(b, qa, __fmul_rn(vd.x, g.id[1]), wi, wa[r][H], yl ? ya[H + r + 1] : ya[H + r - 1],
+                              yl ? ya[H + r + 2] : ya[H + r - 2], p0r, p0c.x, d);
+                    qb = face(b, qb, __fmul_rn(vd.y, g.id[1]), wi, wb[r][H], yl ? yb[H + r + 1] : yb[H + r - 1],
+                              yl ? yb[H + r + 2] : yb[H + r - 2], p0r + 1, p0c.y, d);
+                }
+                if (!ADJ && z == sz && y + r == sy) {  // forward_IO's injection at the shot's cell
+                    const int sx = __ldg(src) + g.pml;
+                    const float inj = inject(sa.wav, g.dt, model_velocity(g, b.vel + (long long)sample * g.ncell, src));
+                    if (x == sx) qa = __fadd_rn(qa, inj);
+                    if (x + 1 == sx) qb = __fadd_rn(qb, inj);
+                }
+                store2<EDGE, false>(p2 + r * g.pitch, qa, qb, ia, ib);
+                if (EDGE) *reinterpret_cast<float2 *>(scratch + r * kBX + 2 * lane) = make_float2(qa, qb);
+                if (stored && yin[r]) {
+                    if (ADJ)
+                        store2<EDGE, false>(Gv + r * g.ipitch, fmaf_rn(svc[r].x, qa, gvc[r].x),
+                                            fmaf_rn(svc[r].y, qb, gvc[r].y), ia, ib);
+                    else
+                        store2<EDGE, true>(sv + r * g.ipitch, __fmul_rn(__fsub_rn(qa, ua), g.idt2),
+                                           __fmul_rn(__fsub_rn(qb, ub), g.idt2), ia, ib);
+                }
+            }
+        }
+        if (EDGE) {  // the x pass on the warp's strip cells, one a lane
+            __syncwarp();
+            for (int i = lane; i < 2 * nx; i += 32) {
+                const int r = i >= nx, c = i - r * nx;
+                const int xc = c < nl ? x0 + c : rx0 + c - nl, at = xc - x0, d = c < nl ? 1 : -1;
+                if (y + r >= g.nty - L) break;
+                const float *p1c = smem + tap * ST::kPitch + (2 * warp + r + H) * ST::kX + ST::kHaloX + at;
+                const float *own = smem + pair0 + (2 * warp + r) * kBX + at;
+                const float *p0g = p0 + r * g.pitch + (xc - x);
+                const float vdc = own[ST::kOwn];
+                const float q = face(b, scratch[r * kBX + at], __fmul_rn(vdc, g.id[0]),
+                                     c < nl ? xc - L : g.ntx - L - 1 - xc, p1c[0], p1c[d], p1c[2 * d], p0g, own[0], d);
+                p2[r * g.pitch + (xc - x)] = q;
+            }
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (lane == 0) mbar_arrive(empty + tap);
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int m = 0; m < 2 * H; ++m) {
+                wa[r][m] = wa[r][m + 1];
+                wb[r][m] = wb[r][m + 1];
+            }
+        pair0 += 2 * ST::kOwn;
+        if (pair0 == ST::kScratch) pair0 = ST::kPairBase;
+        p0 += g.sz;
+        p2 += g.sz;
+        if (sv) sv += ps;
+        if (ADJ && Gv) Gv += ps;
+        if (++tap == ST::kStages) tap = 0;
+        if (++front == ST::kStages) {
+            front = 0;
+            front_phase ^= 1;
+        }
+    }
+    if (!ok) {  // a wait gave up: record it, and let copies in flight land before the block retires
+        if (lane == 0) atomicOr(b.status, 1);
+        for (int i = 0; i < ST::kStages; ++i) mbar_wait_bounded(full + i, 0);
+        for (int i = 0; i < ST::kStages; ++i) mbar_wait_bounded(full + i, 1);
+    }
+}
+
+// One time step of every resident solve.  blockIdx.x = tile (x fastest, then
+// y, then z chunk), then the sampling blocks; blockIdx.y = resident slot.  The
+// maps view the ring as [3 * resident][z][y][x].
+template <int H, bool ADJ>
+__global__ void __launch_bounds__(Stage3<H>::kThreads, kBlocksPerSM)
+    k3_step(const __grid_constant__ Maps3 tm, const __grid_constant__ Geom3 g, const __grid_constant__ Batch3 b,
+            const __grid_constant__ Step3 sa)
+{
+    extern __shared__ __align__(1024) float smem[];
+    const int tiles = g.tiles_x * g.tiles_y;
+    int t = blockIdx.x;
+    if (!ADJ && t >= tiles * sa.chunks) {
+        grid_dependency_wait();
+        grid_launch_dependents();
+        const int slot = blockIdx.y;
+        sample3(g, b, b.ring + ((long long)slot * 3 + (sa.k + 1) % 3) * g.fstride, b.inst0 + slot, sa.sample_it,
+                (t - tiles * sa.chunks) * blockDim.x + threadIdx.x, sa.sample_blocks * blockDim.x);
+        return;
+    }
+    const int tx = t % g.tiles_x;
+    t /= g.tiles_x;
+    const int ty = t % g.tiles_y, cz = t / g.tiles_y;
+    const int x0 = g.L + tx * kBX, y0 = g.L + ty * Stage3<H>::kBY;
+    const int z0 = g.L + cz * sa.planes, z1 = min(z0 + sa.planes, g.ntz - g.L);
+    if (x0 >= g.pml && x0 + kBX <= g.ntx - g.pml)
+        march3<H, ADJ, false>(tm, g, b, sa, smem, x0, y0, z0, z1);
+    else
+        march3<H, ADJ, true>(tm, g, b, sa, smem, x0, y0, z0, z1);
+}
+
+// The receivers of the last step, time index it, in p (ring level `level`).
+__global__ void k3_sample(const Geom3 g, const Batch3 b, int level, int it)
+{
+    const int slot = blockIdx.y;
+    grid_dependency_wait();
+    sample3(g, b, b.ring + ((long long)slot * 3 + level) * g.fstride, b.inst0 + slot, it,
+            blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // Adjoint IO of step k (time it): residual injection (syn - obs, the
@@ -294,13 +524,15 @@ __global__ void k3_io_fwd(const Geom3 g, const Batch3 b, int k, int it, float wa
 // cell, with each injection's imaging term.
 __global__ void k3_io_adj(const Geom3 g, const Batch3 b, int k, int it, int snap)
 {
-    const int slot = blockIdx.x;
+    const int slot = blockIdx.y;
     const int inst = b.inst0 + slot;
     const int sample = inst / g.ns, shot = inst - sample * g.ns;
+    grid_dependency_wait();
+    grid_launch_dependents();
     float *p2 = b.ring + (long long)slot * 3 * g.fstride + (long long)((k + 2) % 3) * g.fstride;
     const float *syn = b.syn + ((long long)inst * g.nt + it) * g.nr;
     const float *obs = b.obs + ((long long)shot * g.nt + it) * g.nr;
-    for (int u = threadIdx.x; u < g.nu; u += blockDim.x) {
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < g.nu; u += gridDim.x * blockDim.x) {
         const int r0 = b.uoff[u], r1 = b.uoff[u + 1];
         const int *xyz = b.rec + 3 * b.uidx[r0];
         const long long c = padded_cell(g, xyz);
@@ -330,13 +562,13 @@ __global__ void k3_prepare(const Geom3 g, const float *__restrict__ vel, float *
         const long long r = e - (long long)s * g.fstride;
         const int z = (int)(r / g.sz);
         const long long rz = r - (long long)z * g.sz;
-        const int y = (int)(rz / g.pitch), x = (int)(rz - (long long)y * g.pitch);
+        const int y = (int)(rz / g.pitch), x = (int)(rz - (long long)y * g.pitch) - g.xoff;
         float v = 0.0f;
-        if (x < g.ntx) {
+        if (x >= 0 && x < g.ntx) {
             const int jx = min(max(x - g.pml, 0), g.nx - 1);
             const int jy = min(max(y - g.pml, 0), g.ny - 1);
             const int jz = min(max(z - g.pml, 0), g.nz - 1);
-            v = __fmul_rn(vel[(long long)s * g.istride + ((long long)jy * g.nx + jx) * g.nz + jz], g.dt);
+            v = __fmul_rn(vel[(long long)s * g.ncell + ((long long)jy * g.nx + jx) * g.nz + jz], g.dt);
         }
         vdt[e] = v;
     }
@@ -346,9 +578,9 @@ __global__ void k3_prepare(const Geom3 g, const float *__restrict__ vel, float *
 // FP64): with P^{k+1} = 2P^k - P^{k-1} + v^2 dt^2 (lap P^k + f), dP^{k+1}/dv =
 // (2/v)(P^{k+1} - 2P^k + P^{k-1}) = (2/v) dt^2 * (stored d2p/dt2).
 __global__ void k3_reduce_grad(const Geom3 g, const float *__restrict__ G, const float *__restrict__ vel,
-                               float *__restrict__ grad, int nsamples)
+                               float *__restrict__ grad, int nsamples, const int *status)
 {
-    const long long cells = g.istride;
+    const long long cells = g.ncell;
     const long long total = (long long)nsamples * cells;
     const double coef = 2.0 * ((double)g.nti * (double)g.dt * (double)g.dt);
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
@@ -358,11 +590,11 @@ __global__ void k3_reduce_grad(const Geom3 g, const float *__restrict__ G, const
         const int iz = (int)(m % g.nz);
         const long long r = m / g.nz;
         const int ix = (int)(r % g.nx), iy = (int)(r / g.nx);
-        const long long j = ((long long)iz * g.ny + iy) * g.nx + ix;
+        const long long j = ((long long)iz * g.ny + iy) * g.ipitch + ix + g.ioff;
         double acc = 0.0;
-        for (int shot = 0; shot < g.ns; ++shot) acc += (double)G[((long long)s * g.ns + shot) * cells + j];
+        for (int shot = 0; shot < g.ns; ++shot) acc += (double)G[((long long)s * g.ns + shot) * g.istride + j];
         const double v = (double)vel[e];
-        grad[e] = (float)(coef * acc / v);
+        grad[e] = *status ? __int_as_float(0x7fffffff) : (float)(coef * acc / v);
     }
 }
 
@@ -388,13 +620,14 @@ __global__ void k3_misfit_partial(const float *__restrict__ syn, const float *__
     }
 }
 
-__global__ void k3_misfit_final(const double *__restrict__ part, double *__restrict__ misfit, int nsamples)
+__global__ void k3_misfit_final(const double *__restrict__ part, double *__restrict__ misfit, int nsamples,
+                                const int *status)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nsamples) return;
     double t = 0.0;
     for (int i = 0; i < kMisfitBlocks; ++i) t += part[(long long)s * kMisfitBlocks + i];
-    misfit[s] = 0.5 * t;
+    misfit[s] = *status ? (double)__int_as_float(0x7fffffff) : 0.5 * t;
 }
 
 // ---------------------------------------------------------------------------
@@ -408,6 +641,7 @@ struct Host3 {
 };
 
 static int round_up(int v, int m) { return (v + m - 1) / m * m; }
+static long long round_up64(long long v, long long m) { return (v + m - 1) / m * m; }
 
 static int validate(const gb_fwi3d_params *p, const gb_fwi3d_acq *a)
 {
@@ -445,14 +679,21 @@ static void derive(const gb_fwi3d_params &p, const gb_fwi3d_acq &a, Host3 &h)
     g.pml = p.pml0 + g.L;
     g.nx = p.nx; g.ny = p.ny; g.nz = p.nz;
     g.ntx = p.nx + 2 * g.pml; g.nty = p.ny + 2 * g.pml; g.ntz = p.nz + 2 * g.pml;
-    g.pitch = round_up(g.ntx, kBX);
+    // Column L, where the tiles start, on a 32-byte boundary (a TMA box starts on
+    // a 16-byte one); interior arrays share the alignment, so a lane's two
+    // columns are one 8-byte access in both.
+    g.xoff = round_up(g.L, 8) - g.L;
+    g.pitch = round_up(g.xoff + g.ntx, 8);
     g.sz = (long long)g.pitch * g.nty;
-    g.fstride = g.sz * g.ntz;
-    g.istride = (long long)p.nx * p.ny * p.nz;
+    g.fstride = round_up64(g.sz * g.ntz, 64);
+    g.ioff = (g.xoff + g.pml) % 8;
+    g.ipitch = round_up(g.ioff + p.nx, 8);
+    g.istride = (long long)g.ipitch * p.ny * p.nz;
+    g.ncell = (long long)p.nx * p.ny * p.nz;
     g.nt = p.nt; g.nti = p.nt_interval; g.ns = p.ns; g.nr = p.nr;
-    g.tiles_x = (g.ntx + kBX - 1) / kBX;
-    g.tiles_y = (g.nty + kBY - 1) / kBY;
-    g.chunks_z = (g.ntz + kZC - 1) / kZC;
+    g.tiles_x = (g.ntx - 2 * g.L + kBX - 1) / kBX;
+    const int by = g.L - 1 <= 5 ? 16 : 12;  // Stage3::kBY
+    g.tiles_y = (g.nty - 2 * g.L + by - 1) / by;
     const double d[3] = {p.dx, p.dy, p.dz};
     for (int i = 0; i < 3; ++i) {
         g.id[i] = (float)(1.0 / d[i]);
@@ -484,7 +725,7 @@ static void derive(const gb_fwi3d_params &p, const gb_fwi3d_acq &a, Host3 &h)
 }
 
 struct Layout3 {
-    size_t tab_src, tab_rec, tab_uoff, tab_uidx, tab_w, tab_omw;
+    size_t status, tab_src, tab_rec, tab_uoff, tab_uidx, tab_w, tab_omw;
     size_t vdt, ring, ring2, ckpt, snap, G, syn, part, total;
     int resident, K, nseg, nsnap;
 };
@@ -514,6 +755,7 @@ static Layout3 plan(const Geom3 &g, int nsamples, int resident, bool fwd_only, b
     }
     const size_t f = sizeof(float) * (size_t)g.fstride, fi = sizeof(float) * (size_t)g.istride;
     size_t off = 0;
+    L.status = off;    off = a256(off + sizeof(int));
     L.tab_src = off;   off = a256(off + sizeof(int) * 3 * g.ns);
     L.tab_rec = off;   off = a256(off + sizeof(int) * 3 * g.nr);
     L.tab_uoff = off;  off = a256(off + sizeof(int) * (g.nr + 1));
@@ -544,25 +786,109 @@ static int grid_for(long long n, int block)
     return (int)std::min<long long>((n + block - 1) / block, 152LL * 32);
 }
 
-template <int H>
-static void launch_step(bool adj, const Geom3 &g, const Batch3 &b, int nres, int k, int snap, cudaStream_t st)
+// z chunks of a step of `nres` solves: few (each re-reads 2H planes and fills
+// its pipeline, worth about 2H + 4 planes), but enough blocks for whole waves of
+// the device's 152 x kBlocksPerSM block slots.
+static void plan_chunks(const Geom3 &g, int nres, int H, Step3 &sa)
 {
-    const dim3 grid(g.tiles_x * g.tiles_y * g.chunks_z, nres), block(kBX, kBY);
-    if (adj)
-        k3_step<H, true><<<grid, block, 0, st>>>(g, b, k, snap);
-    else
-        k3_step<H, false><<<grid, block, 0, st>>>(g, b, k, snap);
+    const long long slots = 152LL * kBlocksPerSM, cols = (long long)g.tiles_x * g.tiles_y * nres;
+    const int planes = g.ntz - 2 * g.L;
+    long long best = -1;
+    for (int c = 1; c <= std::max(1, planes / 8); ++c) {
+        const int per = (planes + c - 1) / c, chunks = (planes + per - 1) / per;
+        const long long cost = (cols * chunks + slots - 1) / slots * (per + 2 * H + 4);
+        if (best < 0 || cost < best) {
+            best = cost;
+            sa.chunks = chunks;
+            sa.planes = per;
+        }
+    }
 }
 
-static void step(bool adj, const Geom3 &g, const Batch3 &b, int nres, int k, int snap, cudaStream_t st)
+// Launches with programmatic dependent launch where the previous operation on
+// the stream is a kernel of the same chain (they wait for it themselves).
+template <typename... A>
+static void launch(void (*kernel)(A...), dim3 grid, int threads, int smem, cudaStream_t st, bool overlap, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+    ++t_launches;
+}
+
+template <int H>
+static void launch_step(bool adj, const Maps3 &tm, const Geom3 &g, const Batch3 &b, int nres, Step3 sa,
+                        cudaStream_t st, bool overlap)
+{
+    using ST = Stage3<H>;
+    static_assert(ST::kBY == (H <= 5 ? 16 : 12), "tiles_y of derive()");
+    plan_chunks(g, nres, H, sa);
+    const dim3 grid(g.tiles_x * g.tiles_y * sa.chunks + sa.sample_blocks, nres);
+    if (adj)
+        launch(k3_step<H, true>, grid, ST::kThreads, ST::kSmem, st, overlap, tm, g, b, sa);
+    else
+        launch(k3_step<H, false>, grid, ST::kThreads, ST::kSmem, st, overlap, tm, g, b, sa);
+}
+
+static void step(bool adj, const Maps3 &tm, const Geom3 &g, const Batch3 &b, int nres, const Step3 &sa,
+                 cudaStream_t st, bool overlap)
 {
     switch (g.L - 1) {
-    case 3: launch_step<3>(adj, g, b, nres, k, snap, st); break;
-    case 4: launch_step<4>(adj, g, b, nres, k, snap, st); break;
-    case 5: launch_step<5>(adj, g, b, nres, k, snap, st); break;
-    default: launch_step<6>(adj, g, b, nres, k, snap, st); break;
+    case 3: launch_step<3>(adj, tm, g, b, nres, sa, st, overlap); break;
+    case 4: launch_step<4>(adj, tm, g, b, nres, sa, st, overlap); break;
+    case 5: launch_step<5>(adj, tm, g, b, nres, sa, st, overlap); break;
+    default: launch_step<6>(adj, tm, g, b, nres, sa, st, overlap); break;
     }
-    ++t_launches;
+}
+
+// k3_step's stages may be more than the default 48 KB of shared memory.
+template <int H>
+static bool allow_smem()
+{
+    return cudaFuncSetAttribute(k3_step<H, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Stage3<H>::kSmem) ==
+               cudaSuccess &&
+           cudaFuncSetAttribute(k3_step<H, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Stage3<H>::kSmem) ==
+               cudaSuccess;
+}
+
+static bool prepare_device(int H)
+{
+    switch (H) {
+    case 3: return allow_smem<3>();
+    case 4: return allow_smem<4>();
+    case 5: return allow_smem<5>();
+    default: return allow_smem<6>();
+    }
+}
+
+// A 4-D fp32 tensor map over `depth` fields [depth][z][y][x] with a one-plane
+// box; out-of-range elements read as zero.
+static bool make_map3(CUtensorMap &m, void *base, const Geom3 &g, long long depth, int box_x, int box_y)
+{
+    auto enc = tensor_map_encoder();
+    if (!enc || !ensure_context()) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)g.pitch, (cuuint64_t)g.nty, (cuuint64_t)g.ntz, (cuuint64_t)depth};
+    const cuuint64_t strides[3] = {(cuuint64_t)g.pitch * 4, (cuuint64_t)g.sz * 4, (cuuint64_t)g.fstride * 4};
+    const cuuint32_t box[4] = {(cuuint32_t)box_x, (cuuint32_t)box_y, 1, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+           CUDA_SUCCESS;
+}
+
+static bool make_maps3(Maps3 &m, void *ring, long long fields, void *vdt, int nsamples, const Geom3 &g)
+{
+    const int H = g.L - 1, halo = H <= 4 ? 4 : 8, by = H <= 5 ? 16 : 12;
+    return make_map3(m.p1, ring, g, fields, kBX + 2 * halo, by + 2 * H) && make_map3(m.p0, ring, g, fields, kBX, by) &&
+           make_map3(m.vdt, vdt, g, nsamples, kBX, by);
 }
 
 }  // namespace gbfwi3
@@ -626,6 +952,11 @@ int gb_fwi3d_run(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int nsamples, 
     if (L.total > work_bytes) return GB_FWI2D_ENOMEM;
     cudaStream_t st = (cudaStream_t)stream;
     char *w = (char *)work;
+    Maps3 tm, tm_adj;
+    auto maps = [&](Maps3 &m, size_t ring) { return make_maps3(m, w + ring, 3LL * L.resident, w + L.vdt, nsamples, g); };
+    if (!prepare_device(g.L - 1) || !maps(tm, L.ring)) return GB_FWI2D_ECUDA;
+    if (!fwd_only && !maps(tm_adj, L.ring2)) return GB_FWI2D_ECUDA;
+    cudaMemsetAsync(w + L.status, 0, sizeof(int), st);
     auto up = [&](size_t off, const void *src, size_t n) {
         if (n) cudaMemcpyAsync(w + off, src, n, cudaMemcpyHostToDevice, st);
     };
@@ -652,6 +983,7 @@ int gb_fwi3d_run(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int nsamples, 
     b.uoff = (const int *)(w + L.tab_uoff);
     b.uidx = (const int *)(w + L.tab_uidx);
     b.nsnap = L.nsnap;
+    b.status = (int *)(w + L.status);
     Batch3 ba = b;  // the adjoint's ring
     ba.ring = (float *)(w + L.ring2);
 
@@ -659,13 +991,28 @@ int gb_fwi3d_run(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int nsamples, 
     ++t_launches;
     if (!fwd_only) cudaMemsetAsync(b.G, 0, sizeof(float) * (size_t)g.istride * ninst, st);
     const size_t fb = sizeof(float) * (size_t)g.fstride;
-    const int io_threads = 256;
     float *ck = (float *)(w + L.ckpt);
     const size_t ck_pitch = 2 * (size_t)L.nseg * fb;
     const size_t ring_pitch = 3 * fb;
+    const int io_threads = 256;
+    const int sample_blocks = std::min(64, (g.nr + io_threads - 1) / io_threads);
+    const int inject_blocks = std::min(64, (g.nu + io_threads - 1) / io_threads);
     for (long long i0 = 0; i0 < ninst; i0 += L.resident) {
         const int nres = (int)std::min<long long>(L.resident, ninst - i0);
         b.inst0 = ba.inst0 = (int)i0;
+        bool chained = false;  // the last operation on st is a kernel of this chain
+        // Forward steps: `record` samples the receivers, one step later (the
+        // level of step k - 1 is p1 of step k).
+        auto forward = [&](int k, int snap, bool record) {
+            Step3 sa{};
+            sa.k = k;
+            sa.snap = snap;
+            sa.wav = a->wavelet[k];
+            sa.sample_it = k - 1;
+            sa.sample_blocks = record && k > 0 ? sample_blocks : 0;
+            step(false, tm, g, b, nres, sa, st, chained);
+            chained = true;
+        };
         // forward: data; the stored field (one segment) or the checkpoints
         cudaMemsetAsync(b.ring, 0, 3 * fb * (size_t)nres, st);
         for (int k = 0; k < g.nt; ++k) {
@@ -675,15 +1022,15 @@ int gb_fwi3d_run(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int nsamples, 
                     cudaMemcpy2DAsync((char *)ck + (size_t)(2 * s + hh) * fb, ck_pitch,
                                       (char *)b.ring + (size_t)((k + hh) % 3) * fb, ring_pitch, fb, nres,
                                       cudaMemcpyDeviceToDevice, st);
+                chained = false;
             }
-            const int snap = (!fwd_only && L.nseg == 1 && k % g.nti == 0) ? k / g.nti : -1;
-            step(false, g, b, nres, k, snap, st);
-            k3_io_fwd<<<nres, io_threads, 0, st>>>(g, b, k, k, a->wavelet[k], snap, 1);
-            ++t_launches;
+            forward(k, (!fwd_only && L.nseg == 1 && k % g.nti == 0) ? k / g.nti : -1, true);
         }
+        launch(k3_sample, dim3(sample_blocks, nres), io_threads, 0, st, true, g, b, (g.nt + 1) % 3, g.nt - 1);
         if (fwd_only) continue;
         // adjoint, segment by segment from the last
         cudaMemsetAsync(ba.ring, 0, 3 * fb * (size_t)nres, st);
+        chained = false;
         for (int s = L.nseg - 1; s >= 0; --s) {
             const int k0 = s * L.K, k1 = std::min(k0 + L.K, g.nt);
             if (L.nseg > 1) {
@@ -691,31 +1038,28 @@ int gb_fwi3d_run(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int nsamples, 
                     cudaMemcpy2DAsync((char *)b.ring + (size_t)((k0 + hh) % 3) * fb, ring_pitch,
                                       (char *)ck + (size_t)(2 * s + hh) * fb, ck_pitch, fb, nres,
                                       cudaMemcpyDeviceToDevice, st);
-                for (int k = k0; k < k1; ++k) {
-                    const int snap = k % g.nti == 0 ? (k - k0) / g.nti : -1;
-                    step(false, g, b, nres, k, snap, st);
-                    k3_io_fwd<<<nres, io_threads, 0, st>>>(g, b, k, k, a->wavelet[k], snap, 0);
-                    ++t_launches;
-                }
+                chained = false;
+                for (int k = k0; k < k1; ++k) forward(k, k % g.nti == 0 ? (k - k0) / g.nti : -1, false);
             }
             for (int it = k1 - 1; it >= k0; --it) {
-                const int ka = g.nt - 1 - it;
-                const int snap = it % g.nti == 0 ? (L.nseg == 1 ? it / g.nti : (it - k0) / g.nti) : -1;
-                step(true, g, ba, nres, ka, snap, st);
-                k3_io_adj<<<nres, io_threads, 0, st>>>(g, ba, ka, it, snap);
-                ++t_launches;
+                Step3 sa{};
+                sa.k = g.nt - 1 - it;
+                sa.snap = it % g.nti == 0 ? (L.nseg == 1 ? it / g.nti : (it - k0) / g.nti) : -1;
+                step(true, tm_adj, g, ba, nres, sa, st, chained);
+                chained = true;
+                launch(k3_io_adj, dim3(inject_blocks, nres), io_threads, 0, st, true, g, ba, sa.k, it, sa.snap);
             }
         }
     }
     if (grad && !fwd_only) {
-        k3_reduce_grad<<<grid_for((long long)nsamples * g.istride, 256), 256, 0, st>>>(g, b.G, vel, grad, nsamples);
+        k3_reduce_grad<<<grid_for((long long)nsamples * g.istride, 256), 256, 0, st>>>(g, b.G, vel, grad, nsamples, b.status);
         ++t_launches;
     }
     if (misfit) {
         double *part = (double *)(w + L.part);
         const long long per = (long long)g.ns * g.nt * g.nr;
         k3_misfit_partial<<<dim3(kMisfitBlocks, nsamples), 256, 0, st>>>(b.syn, obs, per, per, part);
-        k3_misfit_final<<<(nsamples + 127) / 128, 128, 0, st>>>(part, misfit, nsamples);
+        k3_misfit_final<<<(nsamples + 127) / 128, 128, 0, st>>>(part, misfit, nsamples, b.status);
         t_launches += 2;
     }
     return cudaGetLastError() == cudaSuccess ? GB_FWI2D_OK : GB_FWI2D_ECUDA;
