@@ -638,17 +638,17 @@ static bool make_step_maps(StepMaps &m, void *base, const Geom &g, long long fie
 
 // The step kernel's variant for launches of `nres` solves of this grid: the
 // tallest tiles that still give the device's 152 x 28 resident warps enough to
-// do.  Tall tiles share their halo rows; short ones shorten the chain of rows
-// that a small launch waits for.  Misfit + gradient, us per step with 16 / 8 /
-// 4 / 2 rows (800 steps): 160 solves of 200x400 (25600 tiles of 16 rows) 76 /
-// 89 / 113 / 178, 16 of 400x800 (7728) 23.1 / 22.4 / 31.8 / 58.2, 40 of
-// 200x400 (6400; 11360 of 8 rows) 21.1 / 18.2 / 24.1 / 43.8, 20 of 200x400
-// (5680 of 8) 17.6 / 13.3 / 13.5 / 22.8, 12 of 110x250 (2664 of 4) 14.0 / 10.3
-// / 7.8 / 6.8, 2 of 32x48 9.4 / 7.8 / 4.8 / 3.3.
+// do.  Tall tiles share their halo rows and their prologue (330 instructions);
+// short ones shorten the chain of rows that a small launch waits for.  Misfit +
+// gradient, us per step with 16 / 8 / 4 rows (800 steps): 160 solves of 200x400
+// (25600 tiles of 16 rows) 70 / 82 / 102, 16 of 400x800 (7728) 23.0 / 22.2 / 30,
+// 40 of 200x400 (6400; 11360 of 8 rows) 21.2 / 17.5 / 22.3, 20 of 200x400 (5680
+// of 8) 17.8 / 13.3 / 12.7, 30 of 120x250 (4950 of 8) 18.0 / 13.5 / 12.5; with 4
+// / 2 rows, 12 of 110x250 (2664 of 4) 7.8 / 6.4, 2 of 32x48 4.8 / 3.5.
 static int step_variant_for(const Geom &g, long long nres)
 {
-    if (nres * step_tiles(g, 16) >= 7300) return 0;
-    if (nres * step_tiles(g, 8) >= 5000) return 1;
+    if (nres * step_tiles(g, 16) >= 9000) return 0;
+    if (nres * step_tiles(g, 8) >= 7500) return 1;
     return nres * step_tiles(g, 4) >= 5000 ? 2 : 3;
 }
 
@@ -827,6 +827,7 @@ static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStre
     Geom g = c.d->g;
     const int K = c.L.ckpt_k, nseg = c.L.ckpt_nseg;
     g.nt_save = K / g.nti;  // snapshot slots per resident solve: one segment's
+    b.tl.stored = (long long)g.nt_save * g.pstride;
     float *ring = (float *)(c.work + c.L.ring);
     float *ring2 = (float *)(c.work + c.L.ring2);
     float *ck = (float *)(c.work + c.L.ckpt);
@@ -979,9 +980,12 @@ static long long enqueue_exact(const Call &c, cudaStream_t st)
     b.coef = c.tab.coef;
     b.blend_fp32 = c.d->blend_fp32 ? 1 : 0;
     b.status = status;
+    const int rows = kStepVariants[c.variant].rows;
+    b.tl = make_tiling(g, rows, 3, ninst);
     Batch bs = b;  // forward steps writing into the store
     bs.ring = store;
     bs.levels = levels;
+    bs.tl = make_tiling(g, rows, levels, ninst);
     ExactBatch x;
     x.vdt = vdt;
     x.abeta = abeta;
@@ -1115,6 +1119,7 @@ static long long enqueue(const Call &c, cudaStream_t st)
     b.slot0 = 0;
     b.levels = 3;
     b.tm_slot0 = 0;
+    if (!g.pstd) b.tl = make_tiling(g, kStepVariants[c.variant].rows, 3, ninst);
     const StepMaps &maps = c.maps;
 
     const int wave = plain ? 1 : c.L.resident;
@@ -1518,6 +1523,7 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
                 P.inst0 = pc.inst0;
                 P.tm_slot0 = slots;
                 P.nres = pc.r;
+                P.by_ns = make_divisor(f.ninst * g.ns < (1LL << 32) ? g.ns : 1);
                 P.first_block = blocks;
                 A.first[q] = blocks;
                 slots += pc.r;
@@ -1540,6 +1546,7 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
             A.imaging = imaging ? 1 : 0;
             A.store = fwd_only ? 0 : 1;
             A.npieces = (int)l.pieces.size();
+            A.tl = make_tiling(g0, kStepVariants[l.variant].rows, 3, 1);
             // Launches of at least kSplitMinResident solves run as two halves on
             // two streams, so the tail of one half's step overlaps the other's.
             l.split = side != nullptr && slots >= kSplitMinResident;

@@ -61,6 +61,33 @@ struct Geom {
     float fd[8];
 };
 
+// Division by a launch constant d: n / d as the high word of n * (2^32 / d + 1),
+// exact for 0 <= n with n * d < 2^32.
+struct Divisor {
+    uint32_t m;  // 0: d = 1
+    __host__ __device__ __forceinline__ int quotient(int n) const
+    {
+#if defined(__CUDA_ARCH__)
+        return m ? (int)__umulhi((uint32_t)n, m) : n;
+#else
+        return m ? (int)(((uint64_t)(uint32_t)n * m) >> 32) : n;
+#endif
+    }
+};
+inline Divisor make_divisor(int d) { return Divisor{d <= 1 ? 0u : (uint32_t)((1ull << 32) / (uint32_t)d + 1)}; }
+
+// How a launch's ranks map to the tiles of a solve (fwi2d_step_tile.inc), worked
+// out once per launch sequence by make_tiling.
+struct Tiling {
+    int top, bottom, rows_s;   // tiles of the top and of the bottom strip, and their rows
+    int strips;                // ranks of the strips' tiles: (top + bottom) * units
+    int narrow, left, narrows; // narrow units of an interior row of tiles, those left of the pairs; their ranks
+    Divisor by_units, by_narrow, by_wides;
+    Divisor by_ns;             // shots: solve -> sample (m = 0 with ns > 1: divide)
+    long long solve;           // floats per resident solve of the ring
+    long long stored;          // ... and of the stored field
+};
+
 // Where the solves of a wave live.  Solve `inst` = sample * ns + shot.
 struct Batch {
     const float *vdt;    // [nsamples][fstride]   padded v*dt per sample
@@ -84,6 +111,7 @@ struct Batch {
     const float *kk;     // pseudo-spectral mode: |k|^2 per padded cell (wavenumber)
     int spec_resident;   // pseudo-spectral mode: solves the real array holds (the half
                          // spectrum starts after them)
+    Tiling tl;           // the FD step's tiles
 };
 
 // Per-launch step data.

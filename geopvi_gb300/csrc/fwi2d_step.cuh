@@ -679,6 +679,9 @@ __global__ void __launch_bounds__(kTileX, MINB)
     b.spec = nullptr;
     b.kk = nullptr;
     b.spec_resident = 0;
+    b.tl = a.tl;
+    b.tl.by_ns = pc.by_ns;
+    b.tl.stored = (long long)pc.nt_save * g.pstride;
     const int it = ADJ ? g.nt - 1 - k : k;
     StepArgs sa = ring_step(k, it, ADJ ? -1 : (it % g.nti) == 0 ? it / g.nti : -1, ADJ ? 0.0f : __ldg(pc.rik + it));
     if (ADJ) adjoint_terms(sa, g.nti, k, 0, g.nt - 1, 0);

@@ -57,6 +57,7 @@ static cudaError_t launch_multi_np(bool adj, const MultiArgs &full, int nact, in
     a.imaging = full.imaging;
     a.store = full.store;
     a.npieces = full.npieces;
+    a.tl = full.tl;
     for (int q = 0; q <= NP; ++q) a.first[q] = full.first[q];
     for (int q = 0; q < NP; ++q) a.piece[q] = full.piece[q];
     cudaLaunchAttribute attr;

@@ -51,6 +51,7 @@ struct PieceArgs {
     int s_iz, r_iz, r_ix0, dr, nr, ds, s_ix0, ns, nt, nti, nt_save;
     int inst0;        // its first solve within the instance
     int tm_slot0;     // its first ring slot among the tensor map's fields
+    Divisor by_ns;    // its Tiling::by_ns
     int nres;         // its solves
     int first_block;  // its first block in the launch
 };
@@ -67,6 +68,7 @@ struct MultiArgsN {
     const BlendCoef *coef;
     int *status;
     int blend_fp32, imaging, store, npieces;
+    Tiling tl;          // of the launch's grid (by_ns, stored: each piece's)
     int first[NP + 1];  // first blocks, ascending; first[npieces] = the blocks of all pieces
     PieceArgs piece[NP];
 };
@@ -85,14 +87,35 @@ template <int H>
 cudaError_t launch_multi_h(bool adj, const MultiArgs &args, int nact, int k, cudaStream_t st, int variant,
                            bool overlap);
 
-// Tiles per solve at R rows per tile (the bands of fwi2d_step_tile.inc), and
-// the widths of the staged boxes.
+// The bands of a solve's rows -- [tile_r0, pml), [pml, ntz - pml), [ntz - pml,
+// tile_r1) -- in tiles of strip_rows(R), R and strip_rows(R) rows.
+inline Tiling make_tiling(const Geom &g, int R, int levels, long long ninst)
+{
+    Tiling t;
+    t.rows_s = strip_rows(R);
+    t.top = (g.pml - g.tile_r0 + t.rows_s - 1) / t.rows_s;
+    t.bottom = (g.tile_r1 - (g.ntz - g.pml) + t.rows_s - 1) / t.rows_s;
+    t.strips = (t.top + t.bottom) * g.units;
+    t.narrow = g.units - 2 * g.wides;
+    t.left = g.wide0 - g.unit0;
+    t.narrows = (g.nz + R - 1) / R * t.narrow;
+    t.by_units = make_divisor(g.units);
+    t.by_narrow = make_divisor(t.narrow);
+    t.by_wides = make_divisor(g.wides);
+    t.by_ns = make_divisor(ninst * g.ns < (1LL << 32) ? g.ns : 1);
+    t.solve = (long long)levels * g.fstride;
+    t.stored = (long long)g.nt_save * g.pstride;
+    return t;
+}
+
+// Tiles per solve at R rows per tile.
 inline int step_tiles(const Geom &g, int R)
 {
-    const int rs = strip_rows(R);
-    const int nt = (g.pml - g.tile_r0 + rs - 1) / rs, nb = (g.tile_r1 - (g.ntz - g.pml) + rs - 1) / rs;
-    return (nt + nb) * g.units + (g.nz + R - 1) / R * (g.units - g.wides);
+    const Tiling t = make_tiling(g, R, 3, 1);
+    return t.strips + t.narrows + (g.nz + R - 1) / R * g.wides;
 }
+
+// Widths of the staged boxes.
 inline int step_box_x(int H, bool wide) { return (wide ? 2 : 1) * kTileX + 2 * (H <= 4 ? 4 : 8); }
 
 }  // namespace gbfwi
