@@ -623,10 +623,50 @@ static const SideStream *side_stream(bool create)
     return &(g_side[key] = ss);
 }
 
-// Waves of at least this many resident solves run as two halves on two
-// streams: each half's steps form their own chain, so the ramp and tail of
-// one half's launches overlap the other half's work.
-constexpr int kSplitMinResident = 32;
+// Waves of at least this many resident solves, or two whose launches have this
+// many tiles, run as two halves on two streams: each half's steps form their own
+// chain, so the ramp and tail of one half's launches overlap the other half's
+// work.  Halves / one chain, us per step of misfit + gradient (1400 steps): 12
+// solves of 120x250 (7900 tiles of 2 rows) 7.8 / 8.4, 20 of 200x400 (11400 of 4)
+// 12.2 / 12.9, 16 of 400x800 (15400 of 8) 18.4 / 20.6, 50 of 60x120 8.5 / 9.7;
+// below, chains of rows bound a launch and halves cost up to 4 %: 3 of 400x800
+// (5800 of 4) 7.8 / 7.7.  Three or four chains: within 2 % of two.
+constexpr int kSplitMinResident = 32, kSplitMinTiles = 6500;
+static bool split_wave(long long nres, long long tiles)
+{
+    return nres >= kSplitMinResident || (nres >= 2 && nres * tiles >= kSplitMinTiles);
+}
+
+// A wave's two halves (or, without a side stream, the whole wave): the solves
+// [0, nlo) on st and [nlo, nres) on the side stream, between fork() and join().
+struct Halves {
+    const SideStream *side;
+    cudaStream_t st;
+    int nlo, nres;
+    Halves(const SideStream *side, cudaStream_t st, int nres)
+        : side(side), st(st), nlo(side ? nres / 2 : nres), nres(nres)
+    {
+    }
+    void fork() const
+    {
+        if (!side) return;
+        cudaEventRecord(side->fork, st);
+        cudaStreamWaitEvent(side->s, side->fork, 0);
+    }
+    void join() const
+    {
+        if (!side) return;
+        cudaEventRecord(side->join, side->s);
+        cudaStreamWaitEvent(st, side->join, 0);
+    }
+    // f(first solve, solves, stream) for each half.
+    template <typename F>
+    void each(F f) const
+    {
+        f(0, nlo, st);
+        if (side) f(nlo, nres - nlo, side->s);
+    }
+};
 
 // The step kernel's maps over `fields` padded fields, boxes of the variant's tiles.
 static bool make_step_maps(StepMaps &m, void *base, const Geom &g, long long fields, int variant)
@@ -636,18 +676,19 @@ static bool make_step_maps(StepMaps &m, void *base, const Geom &g, long long fie
            make_map(m.wide, base, g, fields, step_box_x(H, true), rows);
 }
 
-// The step kernel's variant for launches of `nres` solves of this grid: the
+// The step kernel's variant for waves of `nres` solves of this grid: the
 // tallest tiles that still give the device's 152 x 28 resident warps enough to
 // do.  Tall tiles share their halo rows and their prologue (330 instructions);
-// short ones shorten the chain of rows that a small launch waits for.  Misfit +
-// gradient, us per step with 16 / 8 / 4 rows (800 steps): 160 solves of 200x400
-// (25600 tiles of 16 rows) 70 / 82 / 102, 16 of 400x800 (7728) 23.0 / 22.2 / 30,
-// 40 of 200x400 (6400; 11360 of 8 rows) 21.2 / 17.5 / 22.3, 20 of 200x400 (5680
-// of 8) 17.8 / 13.3 / 12.7, 30 of 120x250 (4950 of 8) 18.0 / 13.5 / 12.5; with 4
-// / 2 rows, 12 of 110x250 (2664 of 4) 7.8 / 6.4, 2 of 32x48 4.8 / 3.5.
+// short ones shorten the chain of rows that a small launch waits for.  Forward +
+// gradient passes, us per step (1400 steps) with 16 / 8 rows: 120 solves of
+// 200x400 (19200 tiles of 16 rows) 102.1 / 108.2, 100 89.0 / 89.7, 80 (12800)
+// 73.9 / 71.3, 24 of 400x800 (11600) 65.1 / 56.4; with 8 / 4 rows: 60 of 120x250
+// (9900 of 8) 34.1 / 38.8, 28 of 200x400 (7950) 32.6 / 31.5, 20 (5680) 29.2 /
+// 24.4; with 4 / 2 rows: 20 of 120x250 (6600 of 4) 19.4 / 25.4, 8 of 200x400
+// (4540) 17.9 / 19.2, 12 of 120x250 (3960) 16.8 / 15.6, 9 of 157x331 17.7 / 15.1.
 static int step_variant_for(const Geom &g, long long nres)
 {
-    if (nres * step_tiles(g, 16) >= 9000) return 0;
+    if (nres * step_tiles(g, 16) >= 15000) return 0;
     if (nres * step_tiles(g, 8) >= 7500) return 1;
     return nres * step_tiles(g, 4) >= 5000 ? 2 : 3;
 }
@@ -822,7 +863,7 @@ static int grid_for(long long n, int threads)
 // running the segment's adjoint steps in a second ring.  The recomputation runs
 // the same kernel on the same inputs, so the snapshots -- and the gradient --
 // are bit for bit those of full storage.
-static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStream_t st)
+static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStream_t st, const SideStream *side)
 {
     Geom g = c.d->g;
     const int K = c.L.ckpt_k, nseg = c.L.ckpt_nseg;
@@ -834,6 +875,17 @@ static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStre
     const size_t fbytes = sizeof(float) * g.fstride;
     const size_t ring_pitch = 3 * fbytes, ck_pitch = 2 * (size_t)nseg * fbytes;
     long long launches = 0;
+    const Halves halves(side, st, nres);
+    // The pair (p0, p1) of step k of the half's solves between their ring and
+    // checkpoint s.
+    auto copy_pair = [&](int k, int s, bool save, int first, int n, cudaStream_t on) {
+        for (int h = 0; h < 2; ++h) {
+            char *c0 = (char *)ck + first * ck_pitch + (size_t)(2 * s + h) * fbytes;
+            char *r0 = (char *)ring + first * ring_pitch + (size_t)((k + h) % 3) * fbytes;
+            cudaMemcpy2DAsync(save ? c0 : r0, save ? ck_pitch : ring_pitch, save ? r0 : c0,
+                              save ? ring_pitch : ck_pitch, fbytes, n, cudaMemcpyDeviceToDevice, on);
+        }
+    };
     auto profile_span = [&](cudaEvent_t &e0, cudaEvent_t &e1) {
         e0 = e1 = nullptr;
         if (c.profile && cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess)
@@ -845,6 +897,14 @@ static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStre
         t_profile.spans.emplace_back(e0, e1);
         t_profile.launches += n;
     };
+    bool prev_step = false;  // the last operation enqueued on the streams is a step
+    auto advance = [&](bool adj, const StepMaps &maps, Batch &on_ring, const StepArgs &sa) {
+        halves.each([&](int first, int n, cudaStream_t on) {
+            on_ring.slot0 = first;
+            launches += step(adj, maps, g, on_ring, n, sa, on, c.variant, prev_step);
+        });
+        prev_step = true;
+    };
     cudaEvent_t e0, e1;
 
     // forward: data only, checkpoints at segment starts
@@ -852,21 +912,16 @@ static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStre
     b.store = 0;
     cudaMemsetAsync(ring, 0, ring_pitch * nres, st);  // all three levels: the steps leave the rim's zeros
     profile_span(e0, e1);
-    bool prev_step = false;  // the last operation enqueued on st is a step
+    halves.fork();
     for (int k = 0; k < g.nt; ++k) {
         if (k % K == 0) {
             prev_step = false;
-            const int s = k / K;
-            cudaMemcpy2DAsync((char *)ck + (size_t)2 * s * fbytes, ck_pitch, (char *)ring + (size_t)(k % 3) * fbytes,
-                              ring_pitch, fbytes, nres, cudaMemcpyDeviceToDevice, st);
-            cudaMemcpy2DAsync((char *)ck + (size_t)(2 * s + 1) * fbytes, ck_pitch,
-                              (char *)ring + (size_t)((k + 1) % 3) * fbytes, ring_pitch, fbytes, nres,
-                              cudaMemcpyDeviceToDevice, st);
+            halves.each([&](int first, int n, cudaStream_t on) { copy_pair(k, k / K, true, first, n, on); });
         }
         const StepArgs sa = ring_step(k, k, -1, c.d->rik[k]);
-        launches += step(false, c.maps, g, b, nres, sa, st, c.variant, prev_step);
-        prev_step = true;
+        advance(false, c.maps, b, sa);
     }
+    halves.join();
     close_span(e0, e1, g.nt);
 
     // adjoint, segment by segment from the last
@@ -875,26 +930,23 @@ static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStre
     ba.ring = ring2;
     b.store = 1;
     profile_span(e0, e1);
+    halves.fork();
     for (int s = nseg - 1; s >= 0; --s) {
         const int k0 = s * K, k1 = std::min(k0 + K, g.nt), snap0 = k0 / g.nti;
-        cudaMemcpy2DAsync((char *)ring + (size_t)(k0 % 3) * fbytes, ring_pitch, (char *)ck + (size_t)2 * s * fbytes,
-                          ck_pitch, fbytes, nres, cudaMemcpyDeviceToDevice, st);
-        cudaMemcpy2DAsync((char *)ring + (size_t)((k0 + 1) % 3) * fbytes, ring_pitch,
-                          (char *)ck + (size_t)(2 * s + 1) * fbytes, ck_pitch, fbytes, nres,
-                          cudaMemcpyDeviceToDevice, st);
+        halves.each([&](int first, int n, cudaStream_t on) { copy_pair(k0, s, false, first, n, on); });
         prev_step = false;
         for (int k = k0; k < k1; ++k) {  // recompute the segment's forward steps, storing them
             const StepArgs sa = ring_step(k, k, (k % g.nti) == 0 ? k / g.nti - snap0 : -1, c.d->rik[k]);
-            launches += step(false, c.maps, g, b, nres, sa, st, c.variant, prev_step);
-            prev_step = true;
+            advance(false, c.maps, b, sa);
         }
         for (int it = k1 - 1; it >= k0; --it) {  // the segment's adjoint steps
             const int k = g.nt - 1 - it;
             StepArgs sa = ring_step(k, it, (it % g.nti) == 0 ? it / g.nti - snap0 : -1, 0.0f);
             adjoint_terms(sa, g.nti, k, g.nt - k1, g.nt - 1 - k0, snap0);
-            launches += step(true, c.maps2, g, ba, nres, sa, st, c.variant, prev_step);
+            advance(true, c.maps2, ba, sa);
         }
     }
+    halves.join();
     close_span(e0, e1, 2LL * g.nt);
     return launches;
 }
@@ -1125,14 +1177,15 @@ static long long enqueue(const Call &c, cudaStream_t st)
     const int wave = plain ? 1 : c.L.resident;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(st, &cs);
-    const SideStream *side = (g.pstd || wave < kSplitMinResident || c.single_stream)
+    const int tiles = g.pstd ? 0 : step_tiles(g, kStepVariants[c.variant].rows);
+    const SideStream *side = (g.pstd || !split_wave(wave, tiles) || c.single_stream)
                                  ? nullptr
                                  : side_stream(cs == cudaStreamCaptureStatusNone);
     const bool ckpt = (c.flags & GB_FWI2D_CHECKPOINT) && !fwd_only;
     for (long long i0 = 0; i0 < ninst && ckpt; i0 += wave) {
         const int nres = (int)std::min<long long>(wave, ninst - i0);
         b.inst0 = (int)i0;
-        launches += enqueue_checkpointed(c, b, nres, st);
+        launches += enqueue_checkpointed(c, b, nres, st, split_wave(nres, tiles) ? side : nullptr);
     }
     for (long long i0 = 0; i0 < ninst && !ckpt; i0 += wave) {
         const int nres = (int)std::min<long long>(wave, ninst - i0);
@@ -1145,25 +1198,18 @@ static long long enqueue(const Call &c, cudaStream_t st)
             cudaEvent_t e0 = nullptr, e1 = nullptr;
             if (c.profile && cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess)
                 cudaEventRecord(e0, st);
-            const bool split = side && nres >= kSplitMinResident;
-            const int nlo = split ? nres / 2 : nres;
-            Batch bhi = b;
-            bhi.slot0 = nlo;
-            if (split) {  // fork: the second half's chain on the side stream
-                cudaEventRecord(side->fork, st);
-                cudaStreamWaitEvent(side->s, side->fork, 0);
-            }
+            const Halves halves(split_wave(nres, tiles) ? side : nullptr, st, nres);
+            halves.fork();
             for (int k = 0; k < g.nt; ++k) {
                 const int it = adj ? g.nt - 1 - k : k;
                 StepArgs sa = ring_step(k, it, (it % g.nti) == 0 ? it / g.nti : -1, adj ? 0.0f : c.d->rik[it]);
                 if (adj) adjoint_terms(sa, g.nti, k, 0, g.nt - 1, 0);
-                launches += step(adj, maps, g, b, nlo, sa, st, c.variant, k > 0);
-                if (split) launches += step(adj, maps, g, bhi, nres - nlo, sa, side->s, c.variant, k > 0);
+                halves.each([&](int first, int n, cudaStream_t s) {
+                    b.slot0 = first;
+                    launches += step(adj, maps, g, b, n, sa, s, c.variant, k > 0);
+                });
             }
-            if (split) {  // join
-                cudaEventRecord(side->join, side->s);
-                cudaStreamWaitEvent(st, side->join, 0);
-            }
+            halves.join();
             if (e1) {
                 cudaEventRecord(e1, st);
                 t_profile.spans.emplace_back(e0, e1);
@@ -1547,9 +1593,7 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
             A.store = fwd_only ? 0 : 1;
             A.npieces = (int)l.pieces.size();
             A.tl = make_tiling(g0, kStepVariants[l.variant].rows, 3, 1);
-            // Launches of at least kSplitMinResident solves run as two halves on
-            // two streams, so the tail of one half's step overlaps the other's.
-            l.split = side != nullptr && slots >= kSplitMinResident;
+            l.split = side != nullptr && split_wave(slots, tiles);
             if (l.split) split_args(A, l.args_hi, slots / 2, g0, fwd_only, tiles);
         }
     }

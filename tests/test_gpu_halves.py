@@ -1,0 +1,35 @@
+"""Waves that run as two halves on two streams give the bits of solves run one at a time.
+
+Halves start at 32 solves, or where a launch of two solves or more has many tiles; the cases lie on both
+sides of it, with an odd number of solves, several waves, and with a checkpointed field.
+"""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# nz, nx, shots, samples, nt, engine options
+CASES = [
+    (40, 60, 11, 3, 90, dict()),                      # 33 small solves
+    (40, 60, 11, 3, 90, dict(checkpoint=True)),
+    (40, 60, 11, 6, 90, dict(max_resident=35)),       # a wave of 35 and one of 31
+    (40, 60, 11, 6, 90, dict(max_resident=35, checkpoint=True)),
+    (300, 420, 7, 1, 45, dict()),                     # 7 solves with many tiles
+    (300, 420, 7, 1, 45, dict(checkpoint=True)),
+]
+
+
+@pytest.mark.parametrize("graph", (False, True))
+@pytest.mark.parametrize("nz,nx,ns,n,nt,kw", CASES)
+def test_halves_match_single_solves(engine_lib, cuda, nz, nx, ns, n, nt, kw, graph):
+    import torch
+    from geopvi_gb300 import workloads
+    from geopvi_gb300.engine import Fwi2dEngine
+    p = workloads.make_params(nz, nx, nt, 1e-3, ns, 12.0, pml0=10)
+    g = torch.Generator(device=cuda).manual_seed(3)
+    vel = (2500 + 200 * torch.randn(n, nz * nx, generator=g, device=cuda)).clamp(1500, 4500)
+    obs = 0.01 * torch.randn(p.data_len, generator=g, device=cuda)
+    one = Fwi2dEngine(p, device=cuda, graph=False, max_resident=1)
+    ref = one.run(vel, obs, want_syn=True)
+    r = Fwi2dEngine(p, device=cuda, graph=graph, **kw).run(vel, obs, want_syn=True)
+    for name in ("syn", "grad", "misfit"):
+        assert torch.equal(getattr(r, name), getattr(ref, name)), name
