@@ -28,6 +28,7 @@
 #include "fwi2d_step_launch.h"
 #include "fwi2d_exact_adjoint.cuh"
 #include "fwi2d_pstd.cuh"
+#include "streams.h"
 
 namespace gbfwi {
 
@@ -591,19 +592,10 @@ static bool make_map(CUtensorMap &m, void *base, const Geom &g, long long depth,
 // First failure status of the launches being enqueued on this thread.
 static thread_local int t_enqueue_error = 0;
 
-// Second stream of the main loop's two-halves schedule, per (device, host
-// thread), with its fork / join events.  Kept for the process (a graph
-// capture records work on it) and freed by gb_fwi2d_release_caches.
-struct SideStream {
-    cudaStream_t s = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-};
 static std::mutex g_side_mutex;
 static std::map<std::pair<int, std::thread::id>, SideStream> g_side;
 
-// This thread's side stream on the current device; created on first use
-// unless `create` is false (a stream being captured by the caller).
-static const SideStream *side_stream(bool create)
+const SideStream *side_stream(bool create)
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
@@ -636,37 +628,6 @@ static bool split_wave(long long nres, long long tiles)
 {
     return nres >= kSplitMinResident || (nres >= 2 && nres * tiles >= kSplitMinTiles);
 }
-
-// A wave's two halves (or, without a side stream, the whole wave): the solves
-// [0, nlo) on st and [nlo, nres) on the side stream, between fork() and join().
-struct Halves {
-    const SideStream *side;
-    cudaStream_t st;
-    int nlo, nres;
-    Halves(const SideStream *side, cudaStream_t st, int nres)
-        : side(side), st(st), nlo(side ? nres / 2 : nres), nres(nres)
-    {
-    }
-    void fork() const
-    {
-        if (!side) return;
-        cudaEventRecord(side->fork, st);
-        cudaStreamWaitEvent(side->s, side->fork, 0);
-    }
-    void join() const
-    {
-        if (!side) return;
-        cudaEventRecord(side->join, side->s);
-        cudaStreamWaitEvent(st, side->join, 0);
-    }
-    // f(first solve, solves, stream) for each half.
-    template <typename F>
-    void each(F f) const
-    {
-        f(0, nlo, st);
-        if (side) f(nlo, nres - nlo, side->s);
-    }
-};
 
 // The step kernel's maps over `fields` padded fields, boxes of the variant's tiles.
 static bool make_step_maps(StepMaps &m, void *base, const Geom &g, long long fields, int variant)

@@ -18,21 +18,25 @@
 // ways; the warps take turns at issuing): p1 with its x and y halo, and p0 and
 // v*dt.  The z windows slide in registers.  The z and y passes are uniform over
 // a warp's row; the x pass, which few of a row's cells need, is done afterwards
-// by as many lanes as there are strip cells, packed.  The rim (cells outside [L, n - L)), which the
-// scheme never changes from zero, is not visited: the ring is cleared once.
+// by as many lanes as there are strip cells, packed; the y and x passes take p0
+// from the stages where its cells lie in the tile.  The rim (cells outside [L, n -
+// L)), which the scheme never changes from zero, is not visited: the ring is
+// cleared once.  A wave's solves run as two halves on two streams (streams.h).
 // Fields are [z][y][x], the first updated column on a 32-byte boundary.  The
 // adjoint runs the same operator backwards; its forward field is stored whole
 // or, with GB_FWI3D_CHECKPOINT, as ceil(sqrt(nt))-step segments recomputed from
 // checkpoints.
 //
-// What bounds it: instructions (470 / 565 per warp and plane of 128 cells,
-// forward / adjoint, of which 124 are the stencil's; schedulers issue on 60 % of
-// their cycles with 16 warps an SM), DRAM at 2.2 TB/s.  Measured on 160^3 cells, 4
-// shots, 200 steps of misfit + gradient: 104 ms with one column a thread reading
-// its 16 x and y taps from global memory (219 instructions per 32 cells), 87 ms
-// with the planes of p1 staged (two columns a lane, 8 rows), 93 ms with two rows a
-// lane and the x pass in place, 79 ms with the x pass packed, 73 ms with tiles of
-// interior columns compiled apart.
+// What bounds it: instructions (425 / 510 per warp and plane of 128 cells,
+// forward / adjoint, of which 68 are the stencil's, two columns at a time;
+// schedulers issue on 57 % of their cycles with 16 warps an SM), DRAM at 3 TB/s.
+// Measured on 160^3 cells, 4 shots, 200 steps of misfit + gradient: 104 ms with one
+// column a thread reading its 16 x and y taps from global memory (219 instructions
+// per 32 cells), 87 ms with the planes of p1 staged (two columns a lane, 8 rows),
+// 93 ms with two rows a lane and the x pass in place, 79 ms with the x pass packed,
+// 73 ms with tiles of interior columns compiled apart, 71.5 ms with packed
+// arithmetic, 70.2 ms with p0 from the stages, 53.5 ms as two halves, 52.6 ms with
+// chunks for halves.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -44,6 +48,7 @@
 #include "../../include/geopvi_fwi2d.h"
 #include "../../include/geopvi_fwi3d.h"
 #include "fd_weights.cuh"
+#include "streams.h"
 #include "tma.cuh"
 
 namespace gbfwi3 {
@@ -84,6 +89,7 @@ struct Batch3 {
     const int *uidx;            // [nr]
     int nsnap;                  // stored steps per resident solve
     int inst0;                  // first solve of the wave
+    int slot0;                  // resident slot of the launch's first solve
     int *status;                // nonzero: a bounded wait gave up, results are set to NaN
 };
 
@@ -172,34 +178,94 @@ __device__ __forceinline__ float model_velocity(const Geom3 &g, const float *vel
     return vel[((long long)xyz[1] * g.nx + xyz[0]) * g.nz + xyz[2]];
 }
 
-// The cell's new level from its taps (x[m], y[m], z[m]: m cells away) before
-// the absorbing passes; u = 2 p1 - p0.
-template <int H>
-__device__ __forceinline__ float update3(const Geom3 &g, const float *x, const float *y, const float *z, float p0c,
-                                         float vd, float *u)
+// Two neighbouring columns' values in one register pair, and the packed
+// arithmetic on them: each half rounds as the scalar instruction does.
+typedef unsigned long long Pair;
+
+__device__ __forceinline__ Pair pair(float a, float b)
 {
-    const float pc = z[0];
-    float lx = __fmul_rn(fd_weight<H>(0), pc), ly = lx, lz = lx;
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 split2(Pair p)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ Pair both(float a) { return pair(a, a); }
+__device__ __forceinline__ Pair add2(Pair a, Pair b)
+{
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b)
+{
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c)
+{
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ Pair shared_pair(const float *p) { return *reinterpret_cast<const Pair *>(p); }
+
+// The two cells' new level before the absorbing passes from their taps: y[m]
+// and z[m] m cells away, x[k] the columns 2 k and 2 k + 1 from the first cell
+// on; u = 2 p1 - p0.
+template <int H>
+__device__ __forceinline__ float2 update3(const Geom3 &g, const Pair *x, const Pair *y, const Pair *z, float2 p0c,
+                                          Pair vd, float2 *u)
+{
+    const Pair pc = z[0];
+    Pair lx = mul2(both(fd_weight<H>(0)), pc), ly = lx, lz = lx;
 #pragma unroll
     for (int m = 1; m <= H; ++m) {
-        lx = fmaf_rn(fd_weight<H>(m), __fadd_rn(x[m], x[-m]), lx);
-        ly = fmaf_rn(fd_weight<H>(m), __fadd_rn(y[m], y[-m]), ly);
-        lz = fmaf_rn(fd_weight<H>(m), __fadd_rn(z[m], z[-m]), lz);
+        const Pair w = both(fd_weight<H>(m));
+        Pair sx;
+        if (m % 2 == 0) {
+            sx = add2(x[m / 2], x[-m / 2]);
+        } else {
+            const float2 r0 = split2(x[m / 2]), r1 = split2(x[m / 2 + 1]), l1 = split2(x[-m / 2 - 1]),
+                         l0 = split2(x[-(m / 2)]);
+            sx = pair(__fadd_rn(r0.y, l1.y), __fadd_rn(r1.x, l0.x));
+        }
+        lx = fma2(w, sx, lx);
+        ly = fma2(w, add2(y[m], y[-m]), ly);
+        lz = fma2(w, add2(z[m], z[-m]), lz);
     }
-    float t = __fmul_rn(lz, g.id2[2]);
-    t = fmaf_rn(ly, g.id2[1], t);
-    t = fmaf_rn(lx, g.id2[0], t);
-    *u = fmaf_rn(2.0f, pc, -p0c);
-    return fmaf_rn(__fmul_rn(vd, vd), t, *u);
+    Pair t = mul2(lz, both(g.id2[2]));
+    t = fma2(ly, both(g.id2[1]), t);
+    t = fma2(lx, both(g.id2[0]), t);
+    const float2 c = split2(pc);
+    *u = make_float2(fmaf_rn(2.0f, c.x, -p0c.x), fmaf_rn(2.0f, c.y, -p0c.y));
+    return split2(fma2(mul2(vd, vd), t, pair(u->x, u->y)));
 }
 
-// One face's blend of a cell along an axis: p0 points at the cell, d leads one
-// cell inward, x1 and x2 are p1 at 1 and 2 cells inward, wi the weight index.
-__device__ __forceinline__ float face(const Batch3 &b, float q, float s, int wi, float pc, float x1, float x2,
-                                      const float *p0, float p0c, long long d)
+// p0 at 0 to 4 cells inward of a cell.
+struct Inward {
+    float p[5];
+};
+__device__ __forceinline__ Inward inward_global(const float *p0, float p0c, long long d)
 {
-    return blend(q, s, __ldg(b.w + wi), __ldg(b.omw + wi), pc, x1, x2, p0c, __ldg(p0 + d), __ldg(p0 + 2 * d),
-                 __ldg(p0 + 3 * d), __ldg(p0 + 4 * d));
+    return Inward{{p0c, __ldg(p0 + d), __ldg(p0 + 2 * d), __ldg(p0 + 3 * d), __ldg(p0 + 4 * d)}};
+}
+__device__ __forceinline__ Inward inward_shared(const float *p0, int d)
+{
+    return Inward{{p0[0], p0[d], p0[2 * d], p0[3 * d], p0[4 * d]}};
+}
+
+// One face's blend of a cell along an axis: x1 and x2 are p1 at 1 and 2 cells
+// inward, wi the weight index.
+__device__ __forceinline__ float face(const Batch3 &b, float q, float s, int wi, float pc, float x1, float x2,
+                                      const Inward &p0)
+{
+    return blend(q, s, __ldg(b.w + wi), __ldg(b.omw + wi), pc, x1, x2, p0.p[0], p0.p[1], p0.p[2], p0.p[3], p0.p[4]);
 }
 
 // Receivers of one resident solve: p1 (the level of time index it) into syn.
@@ -235,7 +301,7 @@ __device__ __forceinline__ void march3(const Maps3 &tm, const Geom3 &g, const Ba
 {
     using ST = Stage3<H>;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + ST::kBarriers), *empty = full + ST::kStages;
-    const int slot = blockIdx.y;
+    const int slot = b.slot0 + blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int inst = b.inst0 + slot;
     const int sample = inst / g.ns, shot = inst - sample * g.ns;
@@ -258,6 +324,8 @@ __device__ __forceinline__ void march3(const Maps3 &tm, const Geom3 &g, const Ba
     // [ntx - pml, ntx - L) cut to it.
     const int xe = min(x0 + kBX, g.ntx - L), lx1 = min(xe, g.pml), rx0 = max(x0, g.ntx - g.pml);
     const int nl = max(0, lx1 - x0), nx = nl + max(0, xe - rx0);
+    // Every p0 that the strips' cells read lies in the tile.
+    const bool strips_in = (nl == 0 || lx1 + 4 <= x0 + kBX) && (xe <= rx0 || rx0 - 4 >= x0);
     float *scratch = smem + ST::kScratch + warp * 2 * kBX;
     bool row[2], yin[2];  // updated, interior
 #pragma unroll
@@ -307,20 +375,16 @@ __device__ __forceinline__ void march3(const Maps3 &tm, const Geom3 &g, const Ba
     }
     const int mine = (2 * warp + H) * ST::kX + ST::kHaloX + 2 * lane;  // this lane's place in a staged plane
 
-    // The z windows: wa, wb[r][H + m] = plane z + m of row r's two columns.  The
+    // The z windows: w[r][H + m] = plane z + m of row r's two columns.  The
     // chunk's first 2H planes only fill them; the first H of those are then free.
-    float wa[2][2 * H + 1], wb[2][2 * H + 1];
+    Pair w[2][2 * H + 1];
 #pragma unroll
     for (int i = 0; i < 2 * H; ++i) {
         // planes beyond the first kStages: one for every stage freed two steps ago
         if (i >= 2 && i < H + 2 && threadIdx.x == 0 && i - 2 + ST::kStages < nplanes) issue(i - 2 + ST::kStages);
         ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(full + i % ST::kStages, (i / ST::kStages) & 1));
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const float2 v = shared2(smem + i % ST::kStages * ST::kPitch + mine + r * ST::kX);
-            wa[r][i] = v.x;
-            wb[r][i] = v.y;
-        }
+        for (int r = 0; r < 2; ++r) w[r][i] = shared_pair(smem + i % ST::kStages * ST::kPitch + mine + r * ST::kX);
         if (i < H) {
             __syncwarp();
             if (lane == 0) mbar_arrive(empty + i % ST::kStages);
@@ -363,61 +427,52 @@ __device__ __forceinline__ void march3(const Maps3 &tm, const Geom3 &g, const Ba
         ok = ok && mbar_wait_bounded(full + front, front_phase);
         const float *pl = smem + tap * ST::kPitch + mine, *pf = smem + front * ST::kPitch + mine;
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const float2 v = shared2(pf + r * ST::kX);
-            wa[r][2 * H] = v.x;
-            wb[r][2 * H] = v.y;
-        }
+        for (int r = 0; r < 2; ++r) w[r][2 * H] = shared_pair(pf + r * ST::kX);
         // The columns' y neighbours: rows -H .. H + 1, the lane's own two at H, H + 1.
-        float ya[2 * H + 2], yb[2 * H + 2];
+        Pair yt[2 * H + 2];
 #pragma unroll
-        for (int m = 0; m < 2 * H + 2; ++m) {
-            if (m == H || m == H + 1) {
-                ya[m] = wa[m - H][H];
-                yb[m] = wb[m - H][H];
-                continue;
-            }
-            const float2 v = shared2(pl + (m - H) * ST::kX);
-            ya[m] = v.x;
-            yb[m] = v.y;
-        }
+        for (int m = 0; m < 2 * H + 2; ++m)
+            yt[m] = m == H || m == H + 1 ? w[m - H][H] : shared_pair(pl + (m - H) * ST::kX);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             constexpr int K = (H + 1) / 2;  // pairs on each side that hold the x taps
-            float xt[4 * K + 2];
+            Pair xt[2 * K + 1];
 #pragma unroll
-            for (int k = -K; k <= K; ++k) {
-                if (k == 0) continue;
-                const float2 v = shared2(pl + r * ST::kX + 2 * k);
-                xt[2 * (K + k)] = v.x;
-                xt[2 * (K + k) + 1] = v.y;
-            }
-            xt[2 * K] = wa[r][H];
-            xt[2 * K + 1] = wb[r][H];
+            for (int k = -K; k <= K; ++k) xt[K + k] = k == 0 ? w[r][H] : shared_pair(pl + r * ST::kX + 2 * k);
             const float *own = smem + pair0 + (2 * warp + r) * kBX + 2 * lane;
-            const float2 p0c = shared2(own), vd = shared2(own + ST::kOwn);
-            float ua, ub;
-            float qa = update3<H>(g, xt + 2 * K, ya + H + r, wa[r] + H, p0c.x, vd.x, &ua);
-            float qb = update3<H>(g, xt + 2 * K + 1, yb + H + r, wb[r] + H, p0c.y, vd.y, &ub);
+            const float2 p0c = shared2(own);
+            const Pair vp = shared_pair(own + ST::kOwn);
+            float2 u;
+            const float2 q2 = update3<H>(g, xt + K, yt + H + r, w[r] + H, p0c, vp, &u);
+            float qa = q2.x, qb = q2.y;
             if (row[r]) {
                 // The absorbing passes: z, then y, then x (at most one face each)
                 const float *p0r = p0 + r * g.pitch;
+                const float2 pc = split2(w[r][H]), vd = split2(vp);
                 if (!zin) {
                     const bool zl = z < g.pml;
                     const int wi = zl ? z - L : g.ntz - L - 1 - z;
                     const long long d = zl ? g.sz : -g.sz;
-                    qa = face(b, qa, __fmul_rn(vd.x, g.id[2]), wi, wa[r][H], zl ? wa[r][H + 1] : wa[r][H - 1],
-                              zl ? wa[r][H + 2] : wa[r][H - 2], p0r, p0c.x, d);
-                    qb = face(b, qb, __fmul_rn(vd.y, g.id[2]), wi, wb[r][H], zl ? wb[r][H + 1] : wb[r][H - 1],
-                              zl ? wb[r][H + 2] : wb[r][H - 2], p0r + 1, p0c.y, d);
+                    const float2 n1 = split2(zl ? w[r][H + 1] : w[r][H - 1]), n2 = split2(zl ? w[r][H + 2] : w[r][H - 2]);
+                    qa = face(b, qa, __fmul_rn(vd.x, g.id[2]), wi, pc.x, n1.x, n2.x, inward_global(p0r, p0c.x, d));
+                    qb = face(b, qb, __fmul_rn(vd.y, g.id[2]), wi, pc.y, n1.y, n2.y, inward_global(p0r + 1, p0c.y, d));
                 }
                 if (!yin[r]) {
                     const int wi = yl ? y + r - L : g.nty - L - 1 - y - r;
-                    const long long d = yl ? g.pitch : -g.pitch;
-                    qa = face(b, qa, __fmul_rn(vd.x, g.id[1]), wi, wa[r][H], yl ? ya[H + r + 1] : ya[H + r - 1],
-                              yl ? ya[H + r + 2] : ya[H + r - 2], p0r, p0c.x, d);
-                    qb = face(b, qb, __fmul_rn(vd.y, g.id[1]), wi, wb[r][H], yl ? yb[H + r + 1] : yb[H + r - 1],
-                              yl ? yb[H + r + 2] : yb[H + r - 2], p0r + 1, p0c.y, d);
+                    const int rr = 2 * warp + r, d = yl ? kBX : -kBX;
+                    Inward ea, eb;
+                    if (yl ? rr + 4 < ST::kBY : rr >= 4) {  // in the tile: staged
+                        ea = inward_shared(own, d);
+                        eb = inward_shared(own + 1, d);
+                    } else {
+                        const long long dg = yl ? g.pitch : -g.pitch;
+                        ea = inward_global(p0r, p0c.x, dg);
+                        eb = inward_global(p0r + 1, p0c.y, dg);
+                    }
+                    const float2 n1 = split2(yl ? yt[H + r + 1] : yt[H + r - 1]),
+                                 n2 = split2(yl ? yt[H + r + 2] : yt[H + r - 2]);
+                    qa = face(b, qa, __fmul_rn(vd.x, g.id[1]), wi, pc.x, n1.x, n2.x, ea);
+                    qb = face(b, qb, __fmul_rn(vd.y, g.id[1]), wi, pc.y, n1.y, n2.y, eb);
                 }
                 if (!ADJ && z == sz && y + r == sy) {  // forward_IO's injection at the shot's cell
                     const int sx = __ldg(src) + g.pml;
@@ -432,8 +487,8 @@ __device__ __forceinline__ void march3(const Maps3 &tm, const Geom3 &g, const Ba
                         store2<EDGE, false>(Gv + r * g.ipitch, fmaf_rn(svc[r].x, qa, gvc[r].x),
                                             fmaf_rn(svc[r].y, qb, gvc[r].y), ia, ib);
                     else
-                        store2<EDGE, true>(sv + r * g.ipitch, __fmul_rn(__fsub_rn(qa, ua), g.idt2),
-                                           __fmul_rn(__fsub_rn(qb, ub), g.idt2), ia, ib);
+                        store2<EDGE, true>(sv + r * g.ipitch, __fmul_rn(__fsub_rn(qa, u.x), g.idt2),
+                                           __fmul_rn(__fsub_rn(qb, u.y), g.idt2), ia, ib);
                 }
             }
         }
@@ -445,10 +500,10 @@ __device__ __forceinline__ void march3(const Maps3 &tm, const Geom3 &g, const Ba
                 if (y + r >= g.nty - L) break;
                 const float *p1c = smem + tap * ST::kPitch + (2 * warp + r + H) * ST::kX + ST::kHaloX + at;
                 const float *own = smem + pair0 + (2 * warp + r) * kBX + at;
-                const float *p0g = p0 + r * g.pitch + (xc - x);
-                const float vdc = own[ST::kOwn];
-                const float q = face(b, scratch[r * kBX + at], __fmul_rn(vdc, g.id[0]),
-                                     c < nl ? xc - L : g.ntx - L - 1 - xc, p1c[0], p1c[d], p1c[2 * d], p0g, own[0], d);
+                const float q = face(b, scratch[r * kBX + at], __fmul_rn(own[ST::kOwn], g.id[0]),
+                                     c < nl ? xc - L : g.ntx - L - 1 - xc, p1c[0], p1c[d], p1c[2 * d],
+                                     strips_in ? inward_shared(own, d)
+                                               : inward_global(p0 + r * g.pitch + (xc - x), own[0], d));
                 p2[r * g.pitch + (xc - x)] = q;
             }
         }
@@ -457,10 +512,7 @@ __device__ __forceinline__ void march3(const Maps3 &tm, const Geom3 &g, const Ba
 #pragma unroll
         for (int r = 0; r < 2; ++r)
 #pragma unroll
-            for (int m = 0; m < 2 * H; ++m) {
-                wa[r][m] = wa[r][m + 1];
-                wb[r][m] = wb[r][m + 1];
-            }
+            for (int m = 0; m < 2 * H; ++m) w[r][m] = w[r][m + 1];
         pair0 += 2 * ST::kOwn;
         if (pair0 == ST::kScratch) pair0 = ST::kPairBase;
         p0 += g.sz;
@@ -494,7 +546,7 @@ __global__ void __launch_bounds__(Stage3<H>::kThreads, kBlocksPerSM)
     if (!ADJ && t >= tiles * sa.chunks) {
         grid_dependency_wait();
         grid_launch_dependents();
-        const int slot = blockIdx.y;
+        const int slot = b.slot0 + blockIdx.y;
         sample3(g, b, b.ring + ((long long)slot * 3 + (sa.k + 1) % 3) * g.fstride, b.inst0 + slot, sa.sample_it,
                 (t - tiles * sa.chunks) * blockDim.x + threadIdx.x, sa.sample_blocks * blockDim.x);
         return;
@@ -513,7 +565,7 @@ __global__ void __launch_bounds__(Stage3<H>::kThreads, kBlocksPerSM)
 // The receivers of the last step, time index it, in p (ring level `level`).
 __global__ void k3_sample(const Geom3 g, const Batch3 b, int level, int it)
 {
-    const int slot = blockIdx.y;
+    const int slot = b.slot0 + blockIdx.y;
     grid_dependency_wait();
     sample3(g, b, b.ring + ((long long)slot * 3 + level) * g.fstride, b.inst0 + slot, it,
             blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
@@ -524,7 +576,7 @@ __global__ void k3_sample(const Geom3 g, const Batch3 b, int level, int it)
 // cell, with each injection's imaging term.
 __global__ void k3_io_adj(const Geom3 g, const Batch3 b, int k, int it, int snap)
 {
-    const int slot = blockIdx.y;
+    const int slot = b.slot0 + blockIdx.y;
     const int inst = b.inst0 + slot;
     const int sample = inst / g.ns, shot = inst - sample * g.ns;
     grid_dependency_wait();
@@ -786,17 +838,38 @@ static int grid_for(long long n, int block)
     return (int)std::min<long long>((n + block - 1) / block, 152LL * 32);
 }
 
-// z chunks of a step of `nres` solves: few (each re-reads 2H planes and fills
-// its pipeline, worth about 2H + 4 planes), but enough blocks for whole waves of
-// the device's 152 x kBlocksPerSM block slots.
-static void plan_chunks(const Geom3 &g, int nres, int H, Step3 &sa)
+
+// Waves of at least two solves and this much work (tiles times planes of a step)
+// run as two halves on two streams, so that one half's blocks fill the SMs that
+// the other's last ones leave.  Misfit + gradient, ms, halves / one chain: 8 of
+// 150^3 x 100 steps 44.6 / 51.3, 2 of 100^3 5.7 / 7.5, 3 of 60^3 (3000)
+// with 12th order 6.7 / 6.1.
+constexpr long long kSplitMinWork = 3500;
+static bool split_wave(const Geom3 &g, int nres)
 {
-    const long long slots = 152LL * kBlocksPerSM, cols = (long long)g.tiles_x * g.tiles_y * nres;
+    return nres >= 2 && (long long)nres * g.tiles_x * g.tiles_y * (g.ntz - 2 * g.L) >= kSplitMinWork;
+}
+
+// z chunks of a launch of `nres` solves that has the device's 152 x kBlocksPerSM
+// block slots, or half of them.  A chunk re-reads 2H planes and fills its
+// pipeline, together worth 2H - 1 planes.  A launch's tiles cost unequal amounts:
+// its last wave is about one whole wave too much, and what fits at once lasts as
+// long as its slowest tile, 1.7 times the mean.  Misfit + gradient, ms, halves: 4
+// of 160^3 x 200 steps in 2 / 4 / 6 / 8 chunks 71.5 / 53.5 / 51.4 / 52.0, 8 of
+// 150^3 x 60 in 2 / 4 / 6 29.1 / 26.5 / 26.9, 8 of 60^3 in 2 / 4 / 6 / 8 9.5 / 6.0
+// / 5.1 / 5.3; one chain: 8 of 150^3 in 1 / 4 / 6 44.0 / 32.2 / 30.8, one of 220^3
+// x 100 in 5 / 12 25.7 / 19.5, 3 of 75 x 110 x 61, checkpointed, in 6 (288 blocks)
+// / 7 28.4 / 32.9.
+static void plan_chunks(const Geom3 &g, int nres, int H, bool half, Step3 &sa)
+{
+    const long long slots = 152LL * kBlocksPerSM / (half ? 2 : 1), cols = (long long)g.tiles_x * g.tiles_y * nres;
     const int planes = g.ntz - 2 * g.L;
     long long best = -1;
     for (int c = 1; c <= std::max(1, planes / 8); ++c) {
         const int per = (planes + c - 1) / c, chunks = (planes + per - 1) / per;
-        const long long cost = (cols * chunks + slots - 1) / slots * (per + 2 * H + 4);
+        const long long blocks = cols * chunks;
+        const long long waves = half ? 20 * (blocks + slots) : blocks <= slots ? 34 * slots : 20 * blocks + 17 * slots;
+        const long long cost = waves * (per + 2 * H - 1);
         if (best < 0 || cost < best) {
             best = cost;
             sa.chunks = chunks;
@@ -825,12 +898,12 @@ static void launch(void (*kernel)(A...), dim3 grid, int threads, int smem, cudaS
 }
 
 template <int H>
-static void launch_step(bool adj, const Maps3 &tm, const Geom3 &g, const Batch3 &b, int nres, Step3 sa,
-                        cudaStream_t st, bool overlap)
+static void launch_step(bool adj, const Maps3 &tm, const Geom3 &g, const Batch3 &b, int nres, bool half,
+                        Step3 sa, cudaStream_t st, bool overlap)
 {
     using ST = Stage3<H>;
     static_assert(ST::kBY == (H <= 5 ? 16 : 12), "tiles_y of derive()");
-    plan_chunks(g, nres, H, sa);
+    plan_chunks(g, nres, H, half, sa);
     const dim3 grid(g.tiles_x * g.tiles_y * sa.chunks + sa.sample_blocks, nres);
     if (adj)
         launch(k3_step<H, true>, grid, ST::kThreads, ST::kSmem, st, overlap, tm, g, b, sa);
@@ -838,14 +911,14 @@ static void launch_step(bool adj, const Maps3 &tm, const Geom3 &g, const Batch3 
         launch(k3_step<H, false>, grid, ST::kThreads, ST::kSmem, st, overlap, tm, g, b, sa);
 }
 
-static void step(bool adj, const Maps3 &tm, const Geom3 &g, const Batch3 &b, int nres, const Step3 &sa,
+static void step(bool adj, const Maps3 &tm, const Geom3 &g, const Batch3 &b, int nres, bool half, const Step3 &sa,
                  cudaStream_t st, bool overlap)
 {
     switch (g.L - 1) {
-    case 3: launch_step<3>(adj, tm, g, b, nres, sa, st, overlap); break;
-    case 4: launch_step<4>(adj, tm, g, b, nres, sa, st, overlap); break;
-    case 5: launch_step<5>(adj, tm, g, b, nres, sa, st, overlap); break;
-    default: launch_step<6>(adj, tm, g, b, nres, sa, st, overlap); break;
+    case 3: launch_step<3>(adj, tm, g, b, nres, half, sa, st, overlap); break;
+    case 4: launch_step<4>(adj, tm, g, b, nres, half, sa, st, overlap); break;
+    case 5: launch_step<5>(adj, tm, g, b, nres, half, sa, st, overlap); break;
+    default: launch_step<6>(adj, tm, g, b, nres, half, sa, st, overlap); break;
     }
 }
 
@@ -997,10 +1070,14 @@ int gb_fwi3d_run(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int nsamples, 
     const int io_threads = 256;
     const int sample_blocks = std::min(64, (g.nr + io_threads - 1) / io_threads);
     const int inject_blocks = std::min(64, (g.nu + io_threads - 1) / io_threads);
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(st, &cs);
+    const SideStream *side = split_wave(g, L.resident) ? side_stream(cs == cudaStreamCaptureStatusNone) : nullptr;
     for (long long i0 = 0; i0 < ninst; i0 += L.resident) {
         const int nres = (int)std::min<long long>(L.resident, ninst - i0);
         b.inst0 = ba.inst0 = (int)i0;
-        bool chained = false;  // the last operation on st is a kernel of this chain
+        const Halves halves(split_wave(g, nres) ? side : nullptr, st, nres);
+        bool chained = false;  // the last operation on the streams is a kernel of these chains
         // Forward steps: `record` samples the receivers, one step later (the
         // level of step k - 1 is p1 of step k).
         auto forward = [&](int k, int snap, bool record) {
@@ -1010,46 +1087,56 @@ int gb_fwi3d_run(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int nsamples, 
             sa.wav = a->wavelet[k];
             sa.sample_it = k - 1;
             sa.sample_blocks = record && k > 0 ? sample_blocks : 0;
-            step(false, tm, g, b, nres, sa, st, chained);
+            halves.each([&](int first, int n, cudaStream_t on) {
+                b.slot0 = first;
+                step(false, tm, g, b, n, halves.side != nullptr, sa, on, chained);
+            });
             chained = true;
+        };
+        // The pair (p0, p1) of step k between the ring and checkpoint s.
+        auto copy_pair = [&](int k, int s, bool save) {
+            halves.each([&](int first, int n, cudaStream_t on) {
+                for (int hh = 0; hh < 2; ++hh) {
+                    char *c0 = (char *)ck + first * ck_pitch + (size_t)(2 * s + hh) * fb;
+                    char *r0 = (char *)b.ring + first * ring_pitch + (size_t)((k + hh) % 3) * fb;
+                    cudaMemcpy2DAsync(save ? c0 : r0, save ? ck_pitch : ring_pitch, save ? r0 : c0,
+                                      save ? ring_pitch : ck_pitch, fb, n, cudaMemcpyDeviceToDevice, on);
+                }
+            });
+            chained = false;
         };
         // forward: data; the stored field (one segment) or the checkpoints
         cudaMemsetAsync(b.ring, 0, 3 * fb * (size_t)nres, st);
+        if (!fwd_only) cudaMemsetAsync(ba.ring, 0, 3 * fb * (size_t)nres, st);
+        halves.fork();
         for (int k = 0; k < g.nt; ++k) {
-            if (!fwd_only && L.nseg > 1 && k % L.K == 0) {
-                const int s = k / L.K;
-                for (int hh = 0; hh < 2; ++hh)
-                    cudaMemcpy2DAsync((char *)ck + (size_t)(2 * s + hh) * fb, ck_pitch,
-                                      (char *)b.ring + (size_t)((k + hh) % 3) * fb, ring_pitch, fb, nres,
-                                      cudaMemcpyDeviceToDevice, st);
-                chained = false;
-            }
+            if (!fwd_only && L.nseg > 1 && k % L.K == 0) copy_pair(k, k / L.K, true);
             forward(k, (!fwd_only && L.nseg == 1 && k % g.nti == 0) ? k / g.nti : -1, true);
         }
-        launch(k3_sample, dim3(sample_blocks, nres), io_threads, 0, st, true, g, b, (g.nt + 1) % 3, g.nt - 1);
-        if (fwd_only) continue;
+        halves.each([&](int first, int n, cudaStream_t on) {
+            b.slot0 = first;
+            launch(k3_sample, dim3(sample_blocks, n), io_threads, 0, on, true, g, b, (g.nt + 1) % 3, g.nt - 1);
+        });
         // adjoint, segment by segment from the last
-        cudaMemsetAsync(ba.ring, 0, 3 * fb * (size_t)nres, st);
-        chained = false;
-        for (int s = L.nseg - 1; s >= 0; --s) {
+        for (int s = fwd_only ? -1 : L.nseg - 1; s >= 0; --s) {
             const int k0 = s * L.K, k1 = std::min(k0 + L.K, g.nt);
             if (L.nseg > 1) {
-                for (int hh = 0; hh < 2; ++hh)
-                    cudaMemcpy2DAsync((char *)b.ring + (size_t)((k0 + hh) % 3) * fb, ring_pitch,
-                                      (char *)ck + (size_t)(2 * s + hh) * fb, ck_pitch, fb, nres,
-                                      cudaMemcpyDeviceToDevice, st);
-                chained = false;
+                copy_pair(k0, s, false);
                 for (int k = k0; k < k1; ++k) forward(k, k % g.nti == 0 ? (k - k0) / g.nti : -1, false);
             }
             for (int it = k1 - 1; it >= k0; --it) {
                 Step3 sa{};
                 sa.k = g.nt - 1 - it;
                 sa.snap = it % g.nti == 0 ? (L.nseg == 1 ? it / g.nti : (it - k0) / g.nti) : -1;
-                step(true, tm_adj, g, ba, nres, sa, st, chained);
+                halves.each([&](int first, int n, cudaStream_t on) {
+                    ba.slot0 = first;
+                    step(true, tm_adj, g, ba, n, halves.side != nullptr, sa, on, chained);
+                    launch(k3_io_adj, dim3(inject_blocks, n), io_threads, 0, on, true, g, ba, sa.k, it, sa.snap);
+                });
                 chained = true;
-                launch(k3_io_adj, dim3(inject_blocks, nres), io_threads, 0, st, true, g, ba, sa.k, it, sa.snap);
             }
         }
+        halves.join();
     }
     if (grad && !fwd_only) {
         k3_reduce_grad<<<grid_for((long long)nsamples * g.istride, 256), 256, 0, st>>>(g, b.G, vel, grad, nsamples, b.status);
