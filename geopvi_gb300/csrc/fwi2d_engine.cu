@@ -916,12 +916,12 @@ static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStre
 // be launched programmatically (it waits for that step before reading
 // anything the step writes).
 template <int H>
-static void launch_adjoint_exact(const Call &c, const ExactBatch &x, int nres, int k, int lev1, float rik,
-                                 cudaStream_t st, bool overlap)
+static void launch_adjoint_exact(const Call &c, const ExactBatch &x, int k, int lev1, float rik, cudaStream_t st,
+                                 bool overlap)
 {
     const Geom &g = c.d->g;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(g.pitch / kTileX * ((g.ntz + kTileZ - 1) / kTileZ)), nres);
+    cfg.gridDim = dim3((unsigned)(g.pitch / kTileX * ((g.ntz + kTileZ - 1) / kTileZ) * (long long)x.nres));
     cfg.blockDim = dim3(kAdjThreads);
     cfg.dynamicSmemBytes = AdjShape<H>::kSmem;
     cfg.stream = st;
@@ -934,15 +934,28 @@ static void launch_adjoint_exact(const Call &c, const ExactBatch &x, int nres, i
         t_enqueue_error = GB_FWI2D_ECUDA;
 }
 
-static void adjoint_exact(const Call &c, const ExactBatch &x, int nres, int k, int lev1, float rik, cudaStream_t st,
+static void adjoint_exact(const Call &c, const ExactBatch &x, int k, int lev1, float rik, cudaStream_t st,
                           bool overlap)
 {
     switch (c.d->g.Lc - 1) {
-    case 3: launch_adjoint_exact<3>(c, x, nres, k, lev1, rik, st, overlap); break;
-    case 4: launch_adjoint_exact<4>(c, x, nres, k, lev1, rik, st, overlap); break;
-    case 5: launch_adjoint_exact<5>(c, x, nres, k, lev1, rik, st, overlap); break;
-    default: launch_adjoint_exact<6>(c, x, nres, k, lev1, rik, st, overlap); break;
+    case 3: launch_adjoint_exact<3>(c, x, k, lev1, rik, st, overlap); break;
+    case 4: launch_adjoint_exact<4>(c, x, k, lev1, rik, st, overlap); break;
+    case 5: launch_adjoint_exact<5>(c, x, k, lev1, rik, st, overlap); break;
+    default: launch_adjoint_exact<6>(c, x, k, lev1, rik, st, overlap); break;
     }
+}
+
+// The exact adjoint's plain tiles: every cell in the stencil region and none of a
+// blend's taps (4 cells) within reach.
+static void plain_tiles(const Geom &g, ExactBatch &x)
+{
+    const int lo = g.pml + 4;
+    x.ra = (lo + kTileZ - 1) / kTileZ;
+    x.rb = std::max(x.ra, (g.ntz - lo) / kTileZ);
+    x.ca = (g.xoff + lo + kTileX - 1) / kTileX;
+    x.cb = std::max(x.ca, (g.xoff + g.ntx - lo) / kTileX);
+    const int rows = (g.ntz + kTileZ - 1) / kTileZ, cols = g.pitch / kTileX;
+    if (x.rb == x.ra || x.cb == x.ca || x.rb > rows || x.cb > cols) x.ra = x.rb = x.ca = x.cb = 0;
 }
 
 // Exact gradient.  Per wave: the forward pass (data, and either every level
@@ -1017,65 +1030,87 @@ static long long enqueue_exact(const Call &c, cudaStream_t st)
     x.rdx2 = 1.0f / (g.dx * g.dx);
     x.rdz2 = 1.0f / (g.dz * g.dz);
     x.dtdx = g.dt / g.dx;
+    plain_tiles(g, x);
 
-    // prev_step: the last operation enqueued on st is a step kernel, so the
-    // next may be launched programmatically.
+    // prev_step: the last operation enqueued on the streams is a step kernel, so
+    // the next may be launched programmatically.
     bool prev_step = false;
-    // step it with p0 = store level l, p1 = l + 1, p2 = l + 2
-    auto fwd_store = [&](int it, int l, int nres) {
-        StepArgs sa = ring_step(it, it, -1, c.d->rik[it]);
-        sa.l0 = l;
-        sa.l1 = l + 1;
-        sa.l2 = l + 2;
-        launches += step(false, c.maps2, g, bs, nres, sa, st, c.variant, prev_step);
-        prev_step = true;
-    };
-    const int wave = (c.flags & GB_FWI2D_PLAIN) ? 1 : L.resident;
+    const int wave = (c.flags & GB_FWI2D_PLAIN) ? 1 : L.resident, tiles = step_tiles(g, rows);
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(st, &cs);
+    const SideStream *side = (!split_wave(wave, tiles) || c.single_stream)
+                                 ? nullptr
+                                 : side_stream(cs == cudaStreamCaptureStatusNone);
     // The steps leave the rim of the levels they write as it is: zero, once
     // for all waves (later writes to a level never touch its rim).
     cudaMemsetAsync(store, 0, store_pitch * std::min<long long>(wave, ninst), st);
     for (long long i0 = 0; i0 < ninst; i0 += wave) {
         const int nres = (int)std::min<long long>(wave, ninst - i0);
+        const Halves halves(split_wave(nres, tiles) ? side : nullptr, st, nres);
         b.inst0 = bs.inst0 = x.inst0 = (int)i0;
         prev_step = false;
-        if (nseg == 1) {  // every level in the store: P^-1 = P^0 = 0, step it writes level it + 2
-            cudaMemset2DAsync(store, store_pitch, 0, 2 * fbytes, nres, st);
-            for (int it = 0; it < g.nt; ++it) fwd_store(it, it, nres);
-        } else {
-            cudaMemsetAsync(ring, 0, ring_pitch * nres, st);
-            for (int it = 0; it < g.nt; ++it) {
-                if (it % K == 0) {
-                    const int s = it / K;  // the step's (p0, p1) = (P^{it-1}, P^it)
-                    for (int h = 0; h < 2; ++h)
-                        cudaMemcpy2DAsync((char *)ck + (size_t)(2 * s + h) * fbytes, ck_pitch,
-                                          (char *)ring + (size_t)((it + h) % 3) * fbytes, ring_pitch, fbytes, nres,
-                                          cudaMemcpyDeviceToDevice, st);
-                    prev_step = false;
-                }
-                launches += step(false, c.maps, g, b, nres, ring_step(it, it, -1, c.d->rik[it]), st, c.variant,
-                                 prev_step);
-                prev_step = true;
-            }
-        }
+        auto forward = [&](Batch &on_levels, const StepMaps &maps, const StepArgs &sa) {
+            halves.each([&](int first, int n, cudaStream_t on) {
+                on_levels.slot0 = first;
+                launches += step(false, maps, g, on_levels, n, sa, on, c.variant, prev_step);
+            });
+            prev_step = true;
+        };
+        // step it with p0 = store level l, p1 = l + 1, p2 = l + 2
+        auto fwd_store = [&](int it, int l) {
+            StepArgs sa = ring_step(it, it, -1, c.d->rik[it]);
+            sa.l0 = l;
+            sa.l1 = l + 1;
+            sa.l2 = l + 2;
+            forward(bs, c.maps2, sa);
+        };
         // lambda^{nt+1} = lambda^{nt+2} = 0, and nu with them (its pad columns stay zero)
         cudaMemsetAsync(lam, 0, 3 * fbytes * (size_t)nres, st);
         cudaMemsetAsync(nu, 0, 3 * fbytes * (size_t)nres, st);
-        prev_step = false;
+        if (nseg == 1) {  // every level in the store: P^-1 = P^0 = 0, step it writes level it + 2
+            cudaMemset2DAsync(store, store_pitch, 0, 2 * fbytes, nres, st);
+            halves.fork();
+            for (int it = 0; it < g.nt; ++it) fwd_store(it, it);
+        } else {
+            cudaMemsetAsync(ring, 0, ring_pitch * nres, st);
+            halves.fork();
+            for (int it = 0; it < g.nt; ++it) {
+                if (it % K == 0) {
+                    const int s = it / K;  // the step's (p0, p1) = (P^{it-1}, P^it)
+                    halves.each([&](int first, int n, cudaStream_t on) {
+                        for (int h = 0; h < 2; ++h)
+                            cudaMemcpy2DAsync((char *)ck + first * ck_pitch + (size_t)(2 * s + h) * fbytes, ck_pitch,
+                                              (char *)ring + first * ring_pitch + (size_t)((it + h) % 3) * fbytes,
+                                              ring_pitch, fbytes, n, cudaMemcpyDeviceToDevice, on);
+                    });
+                    prev_step = false;
+                }
+                forward(b, c.maps, ring_step(it, it, -1, c.d->rik[it]));
+            }
+        }
         for (int s = nseg - 1; s >= 0; --s) {
             const int i0s = s * K, i1s = std::min(i0s + K, g.nt);
             if (nseg > 1) {
                 // the pair (P^{i0s-1}, P^{i0s}) into store levels 0, 1; recompute the segment
-                cudaMemcpy2DAsync(store, store_pitch, (char *)ck + (size_t)(2 * s) * fbytes, ck_pitch, 2 * fbytes,
-                                  nres, cudaMemcpyDeviceToDevice, st);
+                halves.each([&](int first, int n, cudaStream_t on) {
+                    cudaMemcpy2DAsync((char *)store + first * store_pitch, store_pitch,
+                                      (char *)ck + first * ck_pitch + (size_t)(2 * s) * fbytes, ck_pitch, 2 * fbytes,
+                                      n, cudaMemcpyDeviceToDevice, on);
+                });
                 prev_step = false;
-                for (int it = i0s; it <= i1s - 2; ++it) fwd_store(it, it - i0s, nres);
+                for (int it = i0s; it <= i1s - 2; ++it) fwd_store(it, it - i0s);
             }
             for (int k = i1s; k >= i0s + 1; --k) {
-                adjoint_exact(c, x, nres, k, k - i0s, c.d->rik[k - 1], st, prev_step);
+                halves.each([&](int first, int n, cudaStream_t on) {
+                    x.slot0 = first;
+                    x.nres = n;
+                    adjoint_exact(c, x, k, k - i0s, c.d->rik[k - 1], on, prev_step);
+                    ++launches;
+                });
                 prev_step = true;
-                ++launches;
             }
         }
+        halves.join();
     }
     if (c.grad) {
         k_reduce_exact<<<grid_for((long long)c.nsamples * g.nz * g.nx, 256), 256, 0, st>>>(g, gpad, c.grad,

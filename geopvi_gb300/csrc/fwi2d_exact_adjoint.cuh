@@ -47,6 +47,9 @@ struct ExactBatch {
     float rdx2, rdz2;      // 1 / dx^2, 1 / dz^2
     float dtdx;            // dt / dx: d s / d v for s = v dt / dx
     int inst0;
+    int slot0;             // resident slot of the launch's first solve
+    int nres;              // solves of the launch
+    int ra, rb, ca, cb;    // plain tiles: rows [ra, rb) and columns [ca, cb) of tiles
 };
 
 // Planes of ExactBatch::taps for one sample: for the z blend (top / bottom
@@ -155,6 +158,29 @@ __global__ void k_exact_tables(const Geom g, const BlendCoef *coef, const float 
 }
 
 
+// The Laplacian of the staged tile at p.
+template <int H>
+__device__ __forceinline__ float tile_laplacian(const float *p, float rdx2, float rdz2)
+{
+    float lx = fd_weight<H>(0) * p[0], lz = lx;
+#pragma unroll
+    for (int m = 1; m <= H; ++m) {
+        lx += fd_weight<H>(m) * (p[m] + p[-m]);
+        lz += fd_weight<H>(m) * (p[m * kBoxX] + p[-m * kBoxX]);
+    }
+    return lx * rdx2 + lz * rdz2;
+}
+
+// a + the terms of the stencil's transpose beyond the centre's, one by one.
+template <int H>
+__device__ __forceinline__ float add_cross(float a, const float *p, float rdx2, float rdz2)
+{
+#pragma unroll
+    for (int m = 1; m <= H; ++m)
+        a += fd_weight<H>(m) * (rdx2 * (p[m] + p[-m]) + rdz2 * (p[m * kBoxX] + p[-m * kBoxX]));
+    return a;
+}
+
 // Step k of the backward recursion for every cell of every resident solve:
 // lambda^k into lam[k % 3] (and nu = a beta lambda^k beside it), and
 // dJ/dv_j += lambda^k_j * d p2_j / d v_j of forward step k-1, whose inputs
@@ -173,6 +199,15 @@ __global__ void k_exact_tables(const Geom g, const BlendCoef *coef, const float 
 // level P^{k-1} for the Laplacian of d p2 / d v.  Band taps stay global
 // loads.  Tiles entirely in the stencil region and four or more cells away
 // from every band take constants for their cell facts.
+//
+// What bounds it: latency -- a band tile's taps are up to 32 dependent pairs of
+// loads a cell, several times a plain tile's time, and 8 solves of 200x400 are 2.5
+// waves of the 152 x 5 resident blocks.  So the band tiles go first (rank order
+// below) and a wave runs as two halves.  Those 8 solves, 1500 steps of both
+// passes: 42.6 ms with tiles row by row, 35.9 with the band tiles first, 33.7 as
+// halves; 4 / 6 blocks an SM cost 1 / 10 % more.  Sums of FMA would save another 4
+// %, but not the order of the terms: added one by one in FMA, the gradient's error
+// against 64 bits grew from 1.0e-5 to 3.3e-5.
 constexpr int kAdjRowsPerThread = 2;                              // rows r0 and r0 + kTileZ / 2
 constexpr int kAdjThreads = kTileX * kTileZ / kAdjRowsPerThread;  // 256
 constexpr int kAdjMinBlocks = 5;  // resident blocks per SM: each waits on its tiles' copy first
@@ -194,19 +229,37 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
     extern __shared__ __align__(1024) float smem[];
     float *s_nu = smem, *s_p1 = smem + AS::kTile;
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + 2 * AS::kTile);  // [0] nu, [1] P^{k-1}
-    const int slot = blockIdx.y;
-    const int inst = b.inst0 + slot;
-    const int sample = inst / g.ns, shot = inst - sample * g.ns;
-    const int tiles_x = g.pitch / kTileX;
-    const int trow = blockIdx.x / tiles_x, tcol = blockIdx.x - trow * tiles_x;
-    const int col0 = tcol * kTileX, row0 = trow * kTileZ;
+    __shared__ int s_place[4];  // slot, sample, tile row, tile column
     const int lane = threadIdx.x & 31, rr0 = threadIdx.x >> 5;  // tile rows rr0 + q * RS
     if (threadIdx.x == 0) {
+        // Solves vary fastest, then the tiles: those of the top and bottom bands'
+        // rows of tiles, the other tiles with band cells, the plain ones.
+        const int t = blockIdx.x / b.nres, slot = b.slot0 + blockIdx.x - t * b.nres;
+        const int tx = g.pitch / kTileX, pr = b.rb - b.ra, pc = b.cb - b.ca;
+        const int n1 = ((g.ntz + kTileZ - 1) / kTileZ - pr) * tx, n2 = pr * (tx - pc);
+        int r, c;
+        if (t < n1) {
+            r = t / tx, c = t - r * tx;
+            r += r < b.ra ? 0 : pr;
+        } else if (t < n1 + n2) {
+            r = (t - n1) / (tx - pc), c = t - n1 - r * (tx - pc);
+            r += b.ra, c += c < b.ca ? 0 : pc;
+        } else {
+            r = (t - n1 - n2) / pc, c = b.ca + t - n1 - n2 - r * pc;
+            r += b.ra;
+        }
+        s_place[0] = slot;
+        s_place[1] = (b.inst0 + slot) / g.ns;
+        s_place[2] = r;
+        s_place[3] = c;
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
         fence_barrier_init();
     }
     __syncthreads();
+    const int slot = s_place[0], sample = s_place[1], trow = s_place[2], tcol = s_place[3];
+    const int inst = b.inst0 + slot, shot = inst - sample * g.ns;
+    const int col0 = tcol * kTileX, row0 = trow * kTileZ;
     const long long P = g.pitch;
     const float *vdt = b.vdt + (long long)sample * g.fstride;
     float *l_base = b.lam + (long long)slot * 3 * g.fstride;
@@ -222,8 +275,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
     // Block-uniform: every cell of the tile in the stencil region, no blend
     // tap within reach (4 cells), so sten = 1, nb = 0, beta = 1.
     const int ix0 = col0 - g.xoff;
-    const bool plain = ix0 >= g.pml + 4 && ix0 + kTileX <= g.ntx - g.pml - 4 && row0 >= g.pml + 4 &&
-                       row0 + kTileZ <= g.ntz - g.pml - 4;
+    const bool plain = trow >= b.ra && trow < b.rb && tcol >= b.ca && tcol < b.cb;
 
     // The per-sample fields are constant through the call: read them while
     // the previous step drains.
@@ -283,10 +335,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
                 }
             }
             out += 2.0f * l1v[q] + fd_weight<H>(0) * (rdx2 + rdz2) * sn[0];
-            out -= l2v[q];
-#pragma unroll
-            for (int m = 1; m <= H; ++m)
-                out += fd_weight<H>(m) * (rdx2 * (sn[m] + sn[-m]) + rdz2 * (sn[m * kBoxX] + sn[-m * kBoxX]));
+            out = add_cross<H>(out - l2v[q], sn, rdx2, rdz2);
             lam0[j] = out;
             nu0[j] = abv[q] * out;
             outp[q] = out;
@@ -305,13 +354,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
             const int iz = row0 + rr;
             const int j = jp + q * RS * g.pitch;
             const float *sp1 = s_p1 + (rr + H) * kBoxX + sc;
-            float lx = fd_weight<H>(0) * sp1[0], lz = lx;
-#pragma unroll
-            for (int m = 1; m <= H; ++m) {
-                lx += fd_weight<H>(m) * (sp1[m] + sp1[-m]);
-                lz += fd_weight<H>(m) * (sp1[m * kBoxX] + sp1[-m * kBoxX]);
-            }
-            float d = 2.0f * vdv[q] * g.dt * (lx * rdx2 + lz * rdz2);
+            float d = 2.0f * vdv[q] * g.dt * tile_laplacian<H>(sp1, rdx2, rdz2);
             if (iz == g.s_iz && ix == g.s_ix0 + shot * g.ds) d += 2.0f * rik_prev * g.dt * vdv[q];
             gp[j] += out * d;
         }
@@ -352,9 +395,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
         } else {
             out += cj.beta * l1v[q];
         }
-#pragma unroll
-        for (int m = 1; m <= H; ++m)
-            out += fd_weight<H>(m) * (rdx2 * (sn[m] + sn[-m]) + rdz2 * (sn[m * kBoxX] + sn[-m * kBoxX]));
+        out = add_cross<H>(out, sn, rdx2, rdz2);
         if (!plain) {
             // A1^T and A0^T of the blends: cells c whose band's extrapolation
             // reads j, 0..4 steps inward of c, with their tabled taps.
@@ -428,13 +469,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
         float d = 0.0f;
         if (cj.sten) {
             const float *sp1 = s_p1 + (rr + H) * kBoxX + sc;
-            float lx = fd_weight<H>(0) * sp1[0], lz = lx;
-#pragma unroll
-            for (int m = 1; m <= H; ++m) {
-                lx += fd_weight<H>(m) * (sp1[m] + sp1[-m]);
-                lz += fd_weight<H>(m) * (sp1[m * kBoxX] + sp1[-m * kBoxX]);
-            }
-            d += cj.beta * 2.0f * vdv[q] * g.dt * (lx * rdx2 + lz * rdz2);
+            d += cj.beta * 2.0f * vdv[q] * g.dt * tile_laplacian<H>(sp1, rdx2, rdz2);
         }
         if (cj.nb) {
             const float s = vdv[q] * g.rdx;

@@ -53,3 +53,22 @@ def test_halves_3d_match_single_solves(engine_lib, cuda, ns, nsamples, kw):
     r = fwi3d.Fwi3dEngine(p, src, rec, wavelet, device=cuda, **kw).run(vel, obs, want_syn=True)
     for name in ("syn", "grad", "misfit"):
         assert torch.equal(getattr(r, name), getattr(ref, name)), name
+
+
+@pytest.mark.parametrize("nz,nx,ns,n,kw", [
+    (40, 60, 11, 3, dict()),                       # 33 small solves, no plain tile in a row of tiles' width
+    (40, 60, 11, 3, dict(checkpoint=True)),
+    (12, 14, 3, 1, dict()),                        # band tiles only
+    (131, 197, 33, 1, dict(max_resident=33)),      # plain tiles within odd edges
+])
+def test_exact_gradient_halves_match_single_solves(engine_lib, cuda, nz, nx, ns, n, kw):
+    import torch
+    from geopvi_gb300 import workloads
+    from geopvi_gb300.engine import Fwi2dEngine
+    p = workloads.make_params(nz, nx, 60, 1e-3, ns, 12.0, pml0=10)
+    g = torch.Generator(device=cuda).manual_seed(4)
+    vel = (2500 + 200 * torch.randn(n, nz * nx, generator=g, device=cuda)).clamp(1500, 4500)
+    obs = 0.01 * torch.randn(p.data_len, generator=g, device=cuda)
+    ref = Fwi2dEngine(p, device=cuda, graph=False, max_resident=1).run(vel, obs, exact=True)
+    r = Fwi2dEngine(p, device=cuda, **kw).run(vel, obs, exact=True)
+    assert torch.equal(r.grad, ref.grad) and torch.equal(r.misfit, ref.misfit)
