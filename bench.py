@@ -323,7 +323,7 @@ def run_gpu(args):
     ms = e0.elapsed_time(e1)
     step_ms, step_launches = eng.step_profile()
     device_status = eng.status()
-    step_variant = eng.tuned_variant(nsamples)  # -1: the tuner was still trying variants
+    step_variant = eng.tuned_variant(nsamples)  # the engine's rule on sizes
     ms_max = grp.max_seconds(ms / 1e3) * 1e3
     cu_batch = cell_updates_per_sample(p) * nsamples
     value = grp.throughput(args.steps * cu_batch, ms_max / 1e3)

@@ -38,7 +38,7 @@ NUM_STEP_VARIANTS = 4
 
 
 def flag_variant(v: int) -> int:
-    """Force FD step variant v (0-3); 0 in the flags lets the tuner choose."""
+    """Force FD step variant v (0-3); 0 in the flags leaves it to the engine's rule."""
     return (v + 1) << VARIANT_SHIFT
 
 STATIC_SCRATCH_BYTES = 64 << 20

@@ -1268,6 +1268,7 @@ struct FusedLaunch {
     int variant = 0;          // the step kernel's variant (tile rows)
     MultiArgs args;           // the launch's parameter (the first half of its solves when split)
     bool split = false;       // the second half runs as its own launch on the side stream
+    bool aside = false;       // whole, on the side stream
     MultiArgs args_hi;
 };
 
@@ -1527,6 +1528,19 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
         // them), then their stored fields; within the planned bytes, which
         // counted each ring rounded up on its own.
         size_t used = 0;
+        // A wave's launches of different grids do not depend on one another: unless
+        // one is most of the wave and is split, they are shared out between the two
+        // streams by their estimated times (a launch's latency and its cells).  Three
+        // instances of 200x400 and two of 100x200, 4 to 12 solves each: 33.9 ms with
+        // every launch split, 30.0 whole on either
+        // stream; 48 uneven instances (12 waves) 5.8 s either way.
+        auto seconds = [&](const FusedLaunch &l) {
+            double cells = 0.0;
+            for (int j : l.pieces) cells += (double)w.pieces[j].r * fi[w.pieces[j].inst].d.g.fstride;
+            return l.maxnt * (6e-6 + 4e-12 * cells);
+        };
+        double total = 0.0, load[2] = {0.0, 0.0};
+        for (const auto &l : w.launches) total += seconds(l);
         for (auto &l : w.launches) {
             const FusedInst &f0 = fi[w.pieces[l.pieces[0]].inst];
             const Geom &g0 = f0.d.g;
@@ -1589,7 +1603,10 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
             A.store = fwd_only ? 0 : 1;
             A.npieces = (int)l.pieces.size();
             A.tl = make_tiling(g0, kStepVariants[l.variant].rows, 3, 1);
-            l.split = side != nullptr && split_wave(slots, tiles);
+            l.split = side != nullptr && split_wave(slots, tiles) && seconds(l) > 0.7 * total;
+            l.aside = side != nullptr && !l.split && load[1] < load[0];
+            if (l.split) load[0] += seconds(l) / 2, load[1] += seconds(l) / 2;
+            else load[l.aside] += seconds(l);
             if (l.split) split_args(A, l.args_hi, slots / 2, g0, fwd_only, tiles);
         }
     }
@@ -1618,7 +1635,7 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
             if (profile && cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess)
                 cudaEventRecord(e0, st);
             bool forked = false;
-            for (const auto &l : w.launches) forked |= l.split;
+            for (const auto &l : w.launches) forked |= l.split || l.aside;
             if (forked) {  // fork: the second halves' chain on the side stream
                 cudaEventRecord(side->fork, st);
                 cudaStreamWaitEvent(side->s, side->fork, 0);
@@ -1648,7 +1665,8 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
             for (int k = 0; k < w.maxnt; ++k) {
                 for (size_t li = 0; li < w.launches.size(); ++li) {
                     const FusedLaunch &l = w.launches[li];
-                    launch(l.args, nact[li], k, st, started, l.variant);
+                    if (l.aside) launch(l.args, nact[li], k, side->s, started_hi, l.variant);
+                    else launch(l.args, nact[li], k, st, started, l.variant);
                     if (l.split) launch(l.args_hi, nact_hi[li], k, side->s, started_hi, l.variant);
                 }
             }

@@ -34,7 +34,7 @@ def main():
     ap.add_argument("--ns", type=int, default=None)
     ap.add_argument("--nt-interval", type=int, default=None,
                     help="store every n-th step (keeps the stored field small for multi-pass captures)")
-    ap.add_argument("--variant", type=int, default=None, help="force a step-kernel variant (default: the tuner)")
+    ap.add_argument("--variant", type=int, default=None, help="force a step-kernel variant (default: the engine's rule)")
     args = ap.parse_args()
     w = getattr(workloads, args.config)()
     p = w.params.replace(nt=args.nt)

@@ -42,7 +42,9 @@ from .params import Params
 # (f = 0.07: 1000x2000, 8 solves, 218 G cell-updates/s; f = 0.29: 200x400,
 # 200 solves, 166 G; f = 0.91: 16x32, 4000 solves, 85 G), within 7 % of each;
 # the fixed cost is the latency of one small launch (one 200x400 solve per
-# step: ~22 us).
+# step: ~22 us).  Fitted to the one-column step kernel; the present one takes
+# about two thirds of these times and a quarter of the fixed cost.  Plans compare
+# times, so their choice depends on the ratios only.
 CELL_S = 3.78e-12
 STRIP_CELL_S = 8.69e-12
 LAUNCH_OVERHEAD_S = 20e-6
