@@ -1532,8 +1532,8 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
         // one is most of the wave and is split, they are shared out between the two
         // streams by their estimated times (a launch's latency and its cells).  Three
         // instances of 200x400 and two of 100x200, 4 to 12 solves each: 33.9 ms with
-        // every launch split, 30.0 whole on either
-        // stream; 48 uneven instances (12 waves) 5.8 s either way.
+        // every launch split, 30.0 whole on either stream; 48 uneven instances (12
+        // waves) 5.8 s either way.
         auto seconds = [&](const FusedLaunch &l) {
             double cells = 0.0;
             for (int j : l.pieces) cells += (double)w.pieces[j].r * fi[w.pieces[j].inst].d.g.fstride;
