@@ -747,8 +747,10 @@ static int kk_table(const Derived &d, const float **out)
 
 // One pseudo-spectral time step of the wave's nres solves: pack p1, forward
 // transform, times -|k|^2, inverse transform, then the per-cell update and
-// the rest of the step.  Returns the number of this library's kernels.
-static int step_pstd(bool adj, const Geom &g, const Batch &b, int nres, const StepArgs &sa, cudaStream_t st)
+// the rest of the step.  packed: the step before, of this chain and ring, left
+// p1 where the transform reads it.  Returns the number of this library's kernels.
+static int step_pstd(bool adj, const Geom &g, const Batch &b, int nres, const StepArgs &sa, cudaStream_t st,
+                     bool packed)
 {
     cufftHandle fwd, inv;
     const CufftApi *api = cufft_api();
@@ -761,7 +763,7 @@ static int step_pstd(bool adj, const Geom &g, const Batch &b, int nres, const St
     cufftDoubleComplex *half = reinterpret_cast<cufftDoubleComplex *>(
         (char *)b.spec + align256(sizeof(double) * (size_t)n * b.spec_resident));
     const dim3 grid((unsigned)std::min<long long>((n + 255) / 256, 1024), nres);
-    k_pstd_pack<<<grid, 256, 0, st>>>(g, b.ring, (sa.k + 1) % 3, real);
+    if (!packed) k_pstd_pack<<<grid, 256, 0, st>>>(g, b.ring, (sa.k + 1) % 3, real);
     if (api->set_stream(fwd, st) != CUFFT_SUCCESS || api->exec_d2z(fwd, real, half) != CUFFT_SUCCESS)
         t_enqueue_error = GB_FWI2D_ECUDA;
     k_pstd_scale<<<grid, 256, 0, st>>>(g, b.kk, reinterpret_cast<double2 *>(half));
@@ -772,14 +774,14 @@ static int step_pstd(bool adj, const Geom &g, const Batch &b, int nres, const St
         k_step_pstd<true><<<cells, 256, 0, st>>>(g, b, sa, real);
     else
         k_step_pstd<false><<<cells, 256, 0, st>>>(g, b, sa, real);
-    return 3;
+    return packed ? 2 : 3;
 }
 
 // One time step of the wave; returns the number of this library's kernels.
 static int step(bool adj, const StepMaps &m, const Geom &g, const Batch &b, int nres, const StepArgs &sa,
-                cudaStream_t st, int variant, bool overlap = false)
+                cudaStream_t st, int variant, bool overlap = false, bool packed = false)
 {
-    if (g.pstd) return step_pstd(adj, g, b, nres, sa, st);
+    if (g.pstd) return step_pstd(adj, g, b, nres, sa, st, packed);
     cudaError_t e;
     switch (g.Lc - 1) {
     case 3: e = launch_step_h<3>(adj, m, g, b, nres, sa, st, variant, overlap); break;
@@ -859,12 +861,14 @@ static long long enqueue_checkpointed(const Call &c, Batch b, int nres, cudaStre
         t_profile.launches += n;
     };
     bool prev_step = false;  // the last operation enqueued on the streams is a step
+    bool prev_adj = false;   // ... of the adjoint
     auto advance = [&](bool adj, const StepMaps &maps, Batch &on_ring, const StepArgs &sa) {
         halves.each([&](int first, int n, cudaStream_t on) {
             on_ring.slot0 = first;
-            launches += step(adj, maps, g, on_ring, n, sa, on, c.variant, prev_step);
+            launches += step(adj, maps, g, on_ring, n, sa, on, c.variant, prev_step, prev_step && prev_adj == adj);
         });
         prev_step = true;
+        prev_adj = adj;
     };
     cudaEvent_t e0, e1;
 
@@ -1202,7 +1206,7 @@ static long long enqueue(const Call &c, cudaStream_t st)
                 if (adj) adjoint_terms(sa, g.nti, k, 0, g.nt - 1, 0);
                 halves.each([&](int first, int n, cudaStream_t s) {
                     b.slot0 = first;
-                    launches += step(adj, maps, g, b, n, sa, s, c.variant, k > 0);
+                    launches += step(adj, maps, g, b, n, sa, s, c.variant, k > 0, k > 0);
                 });
             }
             halves.join();

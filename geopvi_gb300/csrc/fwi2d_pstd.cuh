@@ -59,10 +59,12 @@ __global__ void k_pstd_scale(const Geom g, const float *__restrict__ kk, double2
 // thread per padded cell: the spectral update, then abc_for_p's blends
 // (top / bottom, then left / right) from the previous levels in global
 // memory, the injection, receivers and snapshot / gradient term exactly as
-// the FD kernel's general sweep does them.
+// the FD kernel's general sweep does them.  It leaves the new level in `real`
+// too, where the next step's transform reads it: k_pstd_pack, one launch of seven
+// and 4 us of 82 a step (4 solves of 100x200), runs only where a chain starts.
 template <bool ADJ>
 __global__ void __launch_bounds__(256) k_step_pstd(const Geom g, const Batch b, const StepArgs sa,
-                                                   const double *__restrict__ real)
+                                                   double *__restrict__ real)
 {
     const int slot = blockIdx.y;
     const int inst = b.inst0 + slot;
@@ -122,6 +124,7 @@ __global__ void __launch_bounds__(256) k_step_pstd(const Geom g, const Batch b, 
         }
     }
     p2[c] = q;
+    real[(long long)slot * n + d] = (double)q;
     if (!ADJ && iz == g.r_iz) {  // forward_IO receiver sampling (:930-938)
         const int ir = receiver_of(g, ix);
         if (ir >= 0) b.syn[((long long)inst * g.nt + sa.it) * g.nr + ir] = q;
