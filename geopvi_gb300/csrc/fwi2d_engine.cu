@@ -210,12 +210,11 @@ static void inverse_square(float y, float *h, float *l)
     *l = (float)(r - (double)*h);
 }
 
-// div2_two_least(y), or infinity where div_two is not exact for the divisor y;
-// cached, as the checks walk a binade.
-static float two_op_least(float y)
+// two_op_least(y), cached, as its checks walk a binade.
+static TwoOpLeast cached_two_op_least(float y)
 {
     static std::mutex m;
-    static std::map<uint32_t, float> cache;
+    static std::map<uint32_t, TwoOpLeast> cache;
     uint32_t key;
     std::memcpy(&key, &y, sizeof key);
     {
@@ -223,7 +222,7 @@ static float two_op_least(float y)
         auto it = cache.find(key);
         if (it != cache.end()) return it->second;
     }
-    const float least = two_op_exact(y) ? div2_two_least(y) : HUGE_VALF;
+    const TwoOpLeast least = two_op_least(y);
     std::lock_guard<std::mutex> lk(m);
     cache[key] = least;
     return least;
@@ -282,9 +281,9 @@ static int derive(const gb_fwi2d_params &p, Derived &d)
     g.rdz = 1.0f / p.dz;
     g.fast_dx = division_is_exact(p.dx) ? 1 : 0;
     g.fast_dz = division_is_exact(p.dz) ? 1 : 0;
-    const float least_x = two_op_least(p.dx), least_z = two_op_least(p.dz);
-    g.lo1 = least_x < HUGE_VALF ? kDivLo : HUGE_VALF;
-    g.lo2 = std::max(least_x, least_z);
+    const TwoOpLeast least_x = cached_two_op_least(p.dx), least_z = cached_two_op_least(p.dz);
+    g.lo1 = least_x.one;
+    g.lo2 = std::max(least_x.two, least_z.two);
     g.two = g.lo2 < HUGE_VALF ? 1 : 0;
     reciprocal_pair(p.dx, &g.rxh, &g.rxl);
     reciprocal_pair(p.dz, &g.rzh, &g.rzl);

@@ -150,15 +150,15 @@ GBX_HD float round_scaled_to_subnormal(float qs, float rs)
 }
 
 // x / y as RN(x*rh + RN(x*rl)), rh = 1/y rounded toward zero and rl = RN(1/y -
-// rh) >= 0: correctly rounded for every x when the host's check of one
-// binade's significands passes for this y (two_op_exact, fwi2d_engine.cu; the
-// method is Brisebarre, Muller & Raina's multiplication by a constant held in
-// two words, 2004) and no term underflows: |x| >= kDivLo, or x = +-0.  rl >= 0
-// keeps the sign of zeros and of infinities.
+// rh) >= 0: correctly rounded for every |x| >= div_two_least(y), and x = +-0,
+// when the host's check of one binade's significands passes for this y
+// (two_op_exact; the method is Brisebarre, Muller & Raina's multiplication by a
+// constant held in two words, 2004).  rl >= 0 keeps the sign of zeros and of
+// infinities.
 GBX_HD float div_two(float x, float rh, float rl) { return gbx_fma(x, rh, gbx_mul(x, rl)); }
 
 // (x / y) / y with both divisions in two operations: valid for x = +-0 and
-// |x| >= kDiv2Lo with y <= 2^20 (the first quotient stays above kDivLo).
+// |x| >= div2_two_least(y).
 GBX_HD float div2_two(float x, float rh, float rl) { return div_two(div_two(x, rh, rl), rh, rl); }
 
 // rh and rl of div_two for a divisor y in [2^-20, 2^20].
@@ -171,11 +171,13 @@ inline void reciprocal_pair(float y, float *rh, float *rl)
     *rl = std::fmax((float)(r - (double)h), 0x1p-149f);  // not 0: an infinite x times rl stays infinite
 }
 
-// Host: every significand of one binade through div_two; a pass holds for
-// every |x| >= kDivLo, since both products and the sum scale with x.
+// Host: every significand of one binade through div_two.  A pass holds for every
+// x from div_two_least(y) on, where both products and the sum scale with x.  A
+// power of two divides by its exact reciprocal, beside which x*rl vanishes.
 inline bool two_op_exact(float y)
 {
     if (!(y >= 0x1p-20f && y <= 0x1p20f)) return false;
+    if ((gbx_bits(y) & 0x7FFFFFu) == 0u) return true;
     float rh, rl;
     reciprocal_pair(y, &rh, &rl);
     for (uint32_t m = 0; m < (1u << 23); ++m) {
@@ -185,22 +187,50 @@ inline bool two_op_exact(float y)
     return true;
 }
 
-// Host: the least |x| for which div2_two(x, rh, rl) is (x / y) / y (y passes
-// two_op_exact).  Where x*rl is subnormal its rounding error is up to 2^-150; if
-// no quotient of the binade moves when x*rl is off by 2^-31 of the quotient
-// (true for divisors of few bits, whose quotients keep away from midpoints),
-// that is harmless for quotients down to 2^-118, not only above kDivLo.
-inline float div2_two_least(float y)
+// Host: whether no quotient of the binade moves when x*rl is off by 2^-31 of it
+// (y passes two_op_exact).  True for divisors of few bits, whose quotients keep
+// away from midpoints.
+inline bool two_op_slack(float y)
 {
+    if ((gbx_bits(y) & 0x7FFFFFu) == 0u) return true;
     float rh, rl;
     reciprocal_pair(y, &rh, &rl);
     for (uint32_t m = 0; m < (1u << 23); ++m) {
         const float x = gbx_from_bits(0x3F800000u | m);
         const float p = gbx_mul(x, rl), e = gbx_mul(gbx_mul(x, rh), 0x1.01p-31f), q = x / y;
-        if (gbx_fma(x, rh, gbx_add(p, e)) != q || gbx_fma(x, rh, gbx_sub(p, e)) != q) return kDiv2Lo;
+        if (gbx_fma(x, rh, gbx_add(p, e)) != q || gbx_fma(x, rh, gbx_sub(p, e)) != q) return false;
     }
-    return std::fmax(0x1p-118f, std::fmin(kDiv2Lo, y * y * 0x1p-117f));
+    return true;
 }
+
+// The least dividends of the two-operation quotients by y: `one` of div_two,
+// `two` of div2_two; infinity where they are not exact.
+struct TwoOpLeast {
+    float one, two;
+};
+
+// Host.  rl is below 2^-23 / y, and however small it happens to be, so x*rl turns
+// subnormal while x and the quotient are far from it; from there on its rounding
+// no longer scales with x but is off by up to 1.5 * 2^-150.  Two ways out: |x| >=
+// 2^-126 / rl keeps x*rl normal; and a divisor with slack stands that error for
+// quotients from 2^-118 on.  div_two_tiny's dividends start at 2^-85: a divisor
+// whose `one` is above that is refused.
+inline TwoOpLeast two_op_least(float y)
+{
+    TwoOpLeast l{HUGE_VALF, HUGE_VALF};
+    if (!two_op_exact(y)) return l;
+    float rh, rl;
+    reciprocal_pair(y, &rh, &rl);
+    const bool slack = two_op_slack(y);
+    const float one = slack ? std::fmax(0x1p-118f, y * 0x1p-117f) : std::nextafter(0x1p-126f / rl, HUGE_VALF);
+    if (one > 0x1p-85f) return l;
+    l.one = one;
+    l.two = std::fmax(one, y * one * 0x1.00001p0f);  // the first quotient is `one` or more
+    if (!slack) l.two = std::fmax(l.two, kDiv2Lo);   // div2_tiny has the rest
+    return l;
+}
+inline float div_two_least(float y) { return two_op_least(y).one; }
+inline float div2_two_least(float y) { return two_op_least(y).two; }
 
 // x / y correctly rounded for every x (y > 0).  On the proved range: the
 // fast path.  Below it (|x| < 2^-100, including subnormals): xs = x * 2^64 is
@@ -269,8 +299,8 @@ GBX_HD float div2_any(float x, float y, float r, int fast)
 
 GBX_COLD float div2_any_cold(float x, float y, float r, int fast) { return div2_any(x, y, r, fast); }
 
-// xs / y for a scaled dividend xs = x * 2^64 (|x| < kDiv2Lo, two_op_exact(y)),
-// rounded as the float x / y is and scaled alike: q = RN(xs / y) where x / y is
+// xs / y for a scaled dividend xs = x * 2^64 (|x| < 1, div_two_least(y) <= 2^-85:
+// x = +-0 or |xs| >= 2^-85), rounded as the float x / y is and scaled alike: q = RN(xs / y) where x / y is
 // normal, |q| >= 2^-62; below that the quotient rounded to the subnormal grid
 // G = 2^-149 * 2^64.  There (|q| + c) - c rounds |q| to even on G, the ulp of
 // [c, 2c); that is the rounding of the true quotient unless q is a midpoint by
@@ -285,7 +315,8 @@ GBX_HD float div_two_tiny(float xs, float y, float rh, float rl)
     return aq >= c ? q : gbx_copysign(h, q);
 }
 
-// (x / y) / y for |x| < kDiv2Lo, zeros included.
+// (x / y) / y for |x| < 1, zeros and subnormals included, down to any divisor that
+// two_op_least accepts.
 GBX_HD float div2_tiny(float x, float y, float rh, float rl)
 {
     return gbx_mul(div_two_tiny(div_two_tiny(gbx_mul(x, 0x1p64f), y, rh, rl), y, rh, rl), 0x1p-64f);

@@ -42,6 +42,33 @@ float harness_div2_least(float y) { return div2_two_least(y); }
 
 int harness_two_op_exact(float y) { return two_op_exact(y) ? 1 : 0; }
 
+// The quotients against IEEE division on every significand of the binades where
+// their ranges meet: div_two and div2_two from their least dividends on, div2_tiny
+// below.  -1: the divisor is refused.
+long long harness_quotients_at_their_bounds(float y)
+{
+    const TwoOpLeast least = two_op_least(y);
+    if (std::isinf(least.one)) return -1;
+    float rh, rl;
+    reciprocal_pair(y, &rh, &rl);
+    long long bad = 0;
+    auto walk = [&](float from, int binades, auto f) {
+        const int k0 = std::ilogb(from);
+        for (int k = k0; k < k0 + binades; ++k)
+            for (uint32_t m = 0; m < (1u << 23); ++m) {
+                const uint32_t bits = ((uint32_t)(127 + k) << 23) | m;
+                float x;
+                std::memcpy(&x, &bits, 4);
+                f(x);
+            }
+    };
+    walk(least.one, 3, [&](float x) { bad += x >= least.one && !same(div_two(x, rh, rl), x / y); });
+    walk(least.two, 2, [&](float x) { bad += x >= least.two && !same(div2_two(x, rh, rl), (x / y) / y); });
+    walk(0.5f * least.two, 2,
+         [&](float x) { bad += x < least.two && !same(div2_tiny(x, y, rh, rl), (x / y) / y); });
+    return bad;
+}
+
 // div2_tiny against (x / y) / y below kDiv2Lo, down to the subnormals.
 long long harness_div2_tiny(float y)
 {

@@ -19,6 +19,7 @@ def harness(tmp_path_factory):
     L.harness_div_two.argtypes, L.harness_div_two.restype = [f, i, i], ll
     L.harness_div2_tiny.argtypes, L.harness_div2_tiny.restype = [f], ll
     L.harness_two_op_exact.argtypes = [f]
+    L.harness_quotients_at_their_bounds.argtypes, L.harness_quotients_at_their_bounds.restype = [f], ll
     L.harness_div2_least.argtypes, L.harness_div2_least.restype = [f], f
     L.harness_mix.argtypes, L.harness_mix.restype = [i, ll, ctypes.c_uint, ctypes.POINTER(ll)], ll
     return L
@@ -56,3 +57,18 @@ def test_mix_matches_the_double_formula(harness, pml0):
     assert harness.harness_mix(pml0, trials, 5 + pml0, ctypes.byref(left)) == 0
     # 5 of 16 trial kinds are tails, subnormals, ties and cancellations that may need the general path
     assert left.value <= 0.35 * trials * pml0
+
+
+# Divisors of few and of many bits: where x times the reciprocal's low word turns subnormal, it no longer scales.
+@pytest.mark.parametrize("y", [10.0, 12.3, 77.7, 9000.3, 25000.7, 0.37, 0.001, 4096.0, 2.0 ** 20])
+def test_quotients_at_their_least_dividends(harness, y):
+    assert harness.harness_quotients_at_their_bounds(y) == 0
+
+
+@pytest.mark.parametrize("y", [12.3, 77.7, 25000.7])
+def test_tails_of_divisors_of_many_bits(harness, y):
+    assert harness.harness_div2_tiny(y) == 0
+
+
+def test_divisors_whose_low_word_leaves_no_room_for_tails_are_refused(harness):
+    assert harness.harness_two_op_exact(2500.3) == 1 and harness.harness_quotients_at_their_bounds(2500.3) == -1
