@@ -268,12 +268,13 @@ __device__ __forceinline__ float face(const Batch3 &b, float q, float s, int wi,
     return blend(q, s, __ldg(b.w + wi), __ldg(b.omw + wi), pc, x1, x2, p0.p[0], p0.p[1], p0.p[2], p0.p[3], p0.p[4]);
 }
 
-// Receivers of one resident solve: p1 (the level of time index it) into syn.
+// Receivers of one resident solve: p1 (the level of time index it) into syn.  The
+// launch before wrote that level, so its loads are coherent ones, after the wait.
 __device__ __forceinline__ void sample3(const Geom3 &g, const Batch3 &b, const float *p, int inst, int it, int first,
                                         int stride)
 {
     float *out = b.syn + ((long long)inst * g.nt + it) * g.nr;
-    for (int r = first; r < g.nr; r += stride) out[r] = __ldg(p + padded_cell(g, b.rec + 3 * r));
+    for (int r = first; r < g.nr; r += stride) out[r] = p[padded_cell(g, b.rec + 3 * r)];
 }
 
 __device__ __forceinline__ float2 shared2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
