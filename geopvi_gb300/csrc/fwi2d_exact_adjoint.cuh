@@ -398,7 +398,8 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
         out = add_cross<H>(out, sn, rdx2, rdz2);
         if (!plain) {
             // A1^T and A0^T of the blends: cells c whose band's extrapolation
-            // reads j, 0..4 steps inward of c, with their tabled taps.
+            // reads j, 0..4 steps inward of c, with their tabled taps.  lam1 is what
+            // the launch before wrote, and this one may overlap it: no read-only loads.
             const float *tz = b.taps + (long long)sample * kTapPlanes * g.fstride;
             const float *tx = tz + (long long)kBandX * g.fstride;
             const long long fs = g.fstride;
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
                     const int cz = iz - kk;
                     if (cz < g.Lc || cz >= g.pml) continue;
                     const long long c = j - kk * P;
-                    if (kk < 3) out += __ldg(tz + kk * fs + c) * __ldg(lam1 + c);
+                    if (kk < 3) out += __ldg(tz + kk * fs + c) * lam1[c];
                     out -= __ldg(tz + (3 + kk) * fs + c) * __ldg(lam2 + c);
                 }
             }
@@ -418,7 +419,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
                     const int cz = iz + kk;
                     if (cz < g.ntz - g.pml || cz >= g.ntz - g.Lc) continue;
                     const long long c = j + kk * P;
-                    if (kk < 3) out += __ldg(tz + kk * fs + c) * __ldg(lam1 + c);
+                    if (kk < 3) out += __ldg(tz + kk * fs + c) * lam1[c];
                     out -= __ldg(tz + (3 + kk) * fs + c) * __ldg(lam2 + c);
                 }
             }
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
                     const int cx = ix - kk;
                     if (cx < g.Lc || cx >= g.pml) continue;
                     const long long c = j - kk;
-                    if (kk < 3) out += __ldg(tx + kk * fs + c) * __ldg(lam1 + c);
+                    if (kk < 3) out += __ldg(tx + kk * fs + c) * lam1[c];
                     out -= __ldg(tx + (3 + kk) * fs + c) * __ldg(lam2 + c);
                 }
             }
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks)
                     const int cx = ix + kk;
                     if (cx < g.ntx - g.pml || cx >= g.ntx - g.Lc) continue;
                     const long long c = j + kk;
-                    if (kk < 3) out += __ldg(tx + kk * fs + c) * __ldg(lam1 + c);
+                    if (kk < 3) out += __ldg(tx + kk * fs + c) * lam1[c];
                     out -= __ldg(tx + (3 + kk) * fs + c) * __ldg(lam2 + c);
                 }
             }

@@ -11,6 +11,8 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 # What each file may read through __ldg: tables and inputs that are constant through a call, and the level before
 # the previous one (p0, lam2), whose writer had finished when the previous launch began.
 READ_ONLY = {
+    "fwi2d_exact_adjoint.cuh": {"ab", "vdt", "b.cells", "tz", "tx", "lam2"},
+    "fwi2d_step.cuh": {"c", "c.c->bl", "cz->bl", "cz", "p", "p0", "vdt", "w.vdt", "pc.rik"},
     "fwi3d_engine.cu": {"p0", "b.w", "b.omw", "src"},
 }
 
