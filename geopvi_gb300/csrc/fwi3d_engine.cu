@@ -509,6 +509,9 @@ __device__ __forceinline__ void march3(const Maps3 &tm, const Geom3 &g, const Ba
             }
         }
         ok = __all_sync(0xffffffffu, ok);
+        // Every lane's reads of the stages, and of scratch, before lane 0's release
+        // (and the next plane's scratch).
+        __syncwarp();
         if (lane == 0) mbar_arrive(empty + tap);
 #pragma unroll
         for (int r = 0; r < 2; ++r)

@@ -27,3 +27,10 @@ def operands(text):
 def test_read_only_loads_are_of_finished_memory(name):
     text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
     assert set(operands(text)) <= READ_ONLY[name]
+
+
+def test_a_stage_is_released_after_the_whole_warp_has_read_it():
+    """Lane 0's arrival lets the copy engine overwrite the stage; a vote orders no memory, a warp barrier does."""
+    lines = [ln.split("//")[0].strip() for ln in open(os.path.join(CSRC, "fwi3d_engine.cu"))]
+    at = [i for i, ln in enumerate(lines) if re.search(r"mbar_arrive\(empty", ln)]
+    assert at and all(lines[i - 1] == "__syncwarp();" for i in at)
