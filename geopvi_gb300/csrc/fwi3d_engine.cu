@@ -686,6 +686,14 @@ __global__ void k3_misfit_final(const double *__restrict__ part, double *__restr
     misfit[s] = *status ? (double)__int_as_float(0x7fffffff) : 0.5 * t;
 }
 
+// The caller's data after a wait that gave up.
+__global__ void k3_data_lost(float *__restrict__ syn, long long n, const int *status)
+{
+    if (*status == 0) return;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+        syn[e] = __int_as_float(0x7fffffff);
+}
+
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
@@ -1152,6 +1160,11 @@ int gb_fwi3d_run(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int nsamples, 
         k3_misfit_partial<<<dim3(kMisfitBlocks, nsamples), 256, 0, st>>>(b.syn, obs, per, per, part);
         k3_misfit_final<<<(nsamples + 127) / 128, 128, 0, st>>>(part, misfit, nsamples, b.status);
         t_launches += 2;
+    }
+    if (syn) {  // after the misfit, which is NaN by the status itself
+        const long long n = ninst * g.nt * g.nr;
+        k3_data_lost<<<grid_for(n, 256), 256, 0, st>>>(syn, n, b.status);
+        ++t_launches;
     }
     return cudaGetLastError() == cudaSuccess ? GB_FWI2D_OK : GB_FWI2D_ECUDA;
 }

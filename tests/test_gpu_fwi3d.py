@@ -170,3 +170,32 @@ def test_posterior_drop_in(engine_lib, cuda, tmp_path):
     ref2 = [O.run(sub, shots[sl2], c.rec, c.wav, v, data[sl2], grad=True) for v in full]
     assert np.allclose(l2.cpu().numpy(), np.array([r[2] for r in ref2]) * scale, rtol=1e-10)
     assert np.array_equal(g2.cpu().numpy(), np.stack([r[1][mask] for r in ref2]).astype(np.float64) * scale)
+
+
+def test_a_wait_that_gave_up_leaves_no_data(engine_lib, cuda):
+    """The status word (first in the workspace) set while the steps run, as a wait that gives up sets it: the data,
+    the misfit and the gradient of that call are NaN, and the next call is whole again."""
+    import time
+    import torch
+    from geopvi_gb300 import fwi3d, workloads
+    p = fwi3d.Fwi3dParams(nx=200, ny=200, nz=200, nt=800, dt=1e-3, pml0=10, Lc=4)
+    rec = np.array([[x, y, 0] for x in range(0, 200, 20) for y in range(0, 200, 20)])
+    eng = fwi3d.Fwi3dEngine(p, np.array([[90, 90, 2], [120, 60, 2]]), rec, workloads.ricker(p.nt, p.dt, 10.0), device=cuda)
+    vel = torch.full((1, p.ncell), 2500.0, device=cuda)
+    small = torch.zeros(2 * p.nt * len(rec), device=cuda)
+    good = eng.run(vel, small, forward_only=True).syn.clone()
+    assert torch.isfinite(good).all()
+    aside, done = torch.cuda.Stream(), torch.cuda.Event()
+    with torch.cuda.stream(aside):
+        torch.zeros(4, dtype=torch.uint8, device=cuda).fill_(1)  # the kernel is loaded now, not beside the run
+    torch.cuda.synchronize()
+    r = eng.run(vel, small, forward_only=True)
+    done.record()
+    time.sleep(0.005)  # past the call's own clearing of the word, far from its end
+    with torch.cuda.stream(aside):
+        eng._work[:4].fill_(1)
+    aside.synchronize()
+    assert not done.query()  # the word was set while the steps ran
+    torch.cuda.synchronize()
+    assert torch.isnan(r.syn).all() and torch.isnan(r.misfit).all()
+    assert torch.equal(eng.run(vel, small, forward_only=True).syn, good)
