@@ -202,12 +202,14 @@ static int column_offset(int ntx, int Lc, int pml)
     return best;
 }
 
-// 1/y^2 in two words (y the float divisor).
+// 1/y^2 in two words of one sign (y the float divisor): an infinite second
+// difference times either keeps its sign.
 static void inverse_square(float y, float *h, float *l)
 {
     const double r = 1.0 / ((double)y * (double)y);
     *h = (float)r;
-    *l = (float)(r - (double)*h);
+    if ((double)*h > r) *h = std::nextafter(*h, 0.0f);
+    *l = std::max((float)(r - (double)*h), 0x1p-149f);
 }
 
 // two_op_least(y), cached, as its checks walk a binade.

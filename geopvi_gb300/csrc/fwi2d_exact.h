@@ -554,4 +554,26 @@ GBX_HD float blend_mix(float a, float q, const BlendCoef &c, int fp32_ok)
     return blend_mix_double(a, q, c.omw);
 }
 
+// blend_mix of the weight with 1 - w = bh + bl, out of line and by value, so that
+// no table address has to stay in registers.
+GBX_COLD float blend_mix_rare(float a, float q, float bh, float bl, int fp32_ok)
+{
+    BlendCoef c{};
+    c.bh = bh;
+    c.bl = bl;
+    c.omw = (double)bh + (double)bl;
+    return blend_mix(a, q, c, fp32_ok);
+}
+
+// RN_f(RN_d(a + (1 - w) q)), 1 - w = bh + bl: one FMA, the split evaluation, or
+// the general one, each where it is proved.  No table entry in sight.
+GBX_HD float blend_mix_values(float a, float q, float bh, float bl, float khi2, float klo2, int fp32_ok)
+{
+    float r = gbx_fma(bh, q, a);
+    if (!blend_one_fma(a, q, khi2, klo2)) {
+        if (!(blend_mix_split(a, q, bh, bl, &r) && fp32_ok)) r = blend_mix_rare(a, q, bh, bl, fp32_ok);
+    }
+    return r;
+}
+
 }  // namespace gbfwi

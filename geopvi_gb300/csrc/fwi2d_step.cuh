@@ -29,12 +29,14 @@
 // Arithmetic: the forward pass is the reference's, operation by operation,
 // with exact shortcuts for its divisions and its double boundary mix
 // (fwi2d_exact.h).  The adjoint's result is a gradient that is compared at
-// 1e-4: it takes the second differences and the extrapolations in the same
-// order, and rounds the rest less often -- the grid constants 1/dx^2, 1/dz^2 in
-// two words, one fused update, no range tests.  (Fusing the second
+// 1e-4: it takes the second differences in the same order and the boundary
+// passes as they are, and rounds the update less often -- the grid constants
+// 1/dx^2, 1/dz^2 in two words, one fused sum.  (Fusing the second
 // differences' sums too saves 16 operations a cell and rounds less, yet its
 // gradient is 1.6 times as far from 64 bits: with the forward pass's own
-// rounding the two fields' errors cancel in part.)
+// rounding the two fields' errors cancel in part.  The boundary mix unproved
+// and its factors without their range test are off by a rounding now and
+// then, and are wrong for infinities.)
 //
 // Measured (200x400, 20 shots, 8 models, 800 steps of misfit + gradient; us per
 // step of 18 M padded cells): 112 with 32x16 tiles in one class and inline exact
@@ -122,11 +124,10 @@ struct AbcCoef {
     float t11, t12, t13;
 };
 
-template <bool ADJ>
 __device__ __forceinline__ AbcCoef abc_coef(const Geom &g, const Geom *gp, float vd)
 {
     float s = div_two(vd, g.rxh, g.rxl);
-    if (!ADJ && !(vd >= g.lo1 || vd == 0.0f)) s = slowness_rare(gp, vd);
+    if (!(vd >= g.lo1 || vd == 0.0f)) s = slowness_rare(gp, vd);
     const float u = fs(2.0f, s);
     return AbcCoef{fm(fm(u, fs(1.0f, s)), 0.5f), fm(s, u), fm(fm(s, fs(s, 1.0f)), 0.5f)};
 }
@@ -135,6 +136,10 @@ __device__ __forceinline__ AbcCoef abc_coef(const Geom &g, const Geom *gp, float
 // the two previous levels along the inward direction, weighted by k.x = w
 // against the current value q.  p1a..p1c = p1 at 0, 1, 2 steps inward;
 // p0a..p0e = p0 at 0..4 steps inward.  `k` holds w, bh, khi2, klo2 of `c`, bl its bl.
+// The adjoint, with its three terms in flight, has no registers to spare for the
+// table's address: its rare path takes its arguments by value.  80 solves of
+// 200x400, 3000 steps of both passes: 249 ms, 256 with the double formula inline
+// in its place, 241 with the split evaluation taken unproved.
 template <bool ADJ>
 __device__ __forceinline__ float blend(float q, const AbcCoef &t, float p1a, float p1b, float p1c, float p0a,
                                        float p0b, float p0c, float p0d, float p0e, const float4 &k,
@@ -148,14 +153,7 @@ __device__ __forceinline__ float blend(float q, const AbcCoef &t, float p1a, flo
     ext = fs(ext, fm(fm(b2, t.t13), p0d));
     ext = fs(ext, fm(fm(t.t13, t.t13), p0e));
     const float a = fm(k.x, ext);
-    if (ADJ) {
-        // As the reference rounds it, but for sums within 2^-9 ulp of a midpoint.
-        // (RN(bh q + RN(bl q + a)) drops bl: w + bh < 1 then damps the strip's
-        // slow components a little every step, 1.5 times the gradient's error.)
-        float r;
-        blend_mix_split(a, q, k.y, bl, &r);
-        return r;
-    }
+    if (ADJ) return blend_mix_values(a, q, k.y, bl, k.z, k.w, fp32_ok);
     // RN_f(RN_d(w ext + (1 - w) q)): one FMA, the split evaluation, or the
     // general one, each where it is proved (fwi2d_exact.h).
     float r = ff(k.y, q, a);
@@ -398,7 +396,7 @@ __device__ __forceinline__ void sweep_z(const Geom &g, const Geom *gp, const Bat
         ++cz;
         win[2 * H] = scol[H * sp];
         float q = update<H, ADJ>(g, gp, scol, win + H, z[0], vd, false);
-        q = blend<ADJ>(q, abc_coef<ADJ>(g, gp, vd), win[H], win[H + 1], win[H + 2], z[0], z[1], z[2], z[3], z[4], k,
+        q = blend<ADJ>(q, abc_coef(g, gp, vd), win[H], win[H + 1], win[H + 2], z[0], z[1], z[2], z[3], z[4], k,
                        bl, cz - 1, b.blend_fp32);
         *p2 = q;
         p2 += st;
@@ -488,7 +486,7 @@ __device__ __forceinline__ void sweep_x(const Geom &g, const Geom *gp, const Bat
         const float p1c = win[H];
         float q = update<H, ADJ>(g, gp, scol, win + H, p0c, vd, !c.sx);
         if (!c.sx) q = c.live ? p1c : 0.0f;  // the rim keeps the previous level, the row padding zero
-        if (c.xs) q = blend_x<ADJ>(c, q, abc_coef<ADJ>(g, gp, vd), scol, p1c, p0c, pi, b);
+        if (c.xs) q = blend_x<ADJ>(c, q, abc_coef(g, gp, vd), scol, p1c, p0c, pi, b);
         *p2 = q;
         p2 += g.pitch;
         if (c.inner) {
@@ -534,7 +532,7 @@ __device__ __forceinline__ void sweep_edge(const Geom &g, const Geom *gp, const 
         float q = update<H, ADJ>(g, gp, scol, win + H, p0c, vd, !(c.sx && sz));
         if (!(c.sx && sz)) q = p1c;  // cells the stencil skips keep the previous level
         if (zb || c.xs) {
-            const AbcCoef t = abc_coef<ADJ>(g, gp, vd);
+            const AbcCoef t = abc_coef(g, gp, vd);
             if (zb) {
                 const BlendCoef *cz = b.coef + (w.dir > 0 ? iz - g.Lc : g.ntz - g.Lc - 1 - iz);
                 const int st = w.st;

@@ -146,4 +146,40 @@ long long harness_mix(int pml0, long long trials, unsigned seed, long long *left
     return bad;
 }
 
+// The adjoint's mix against the double formula (any NaN is a NaN): values of all
+// sizes, cancellations, short significands, sums near a float midpoint, infinities.
+long long harness_mix_values(int pml0, long long trials, unsigned seed, int fp32_ok)
+{
+    std::mt19937_64 rng(seed);
+    std::uniform_real_distribution<double> U(-1.0, 1.0);
+    std::uniform_int_distribution<int> E(-148, 127), M(-(1 << 20), 1 << 20);
+    long long bad = 0;
+    for (int i = 0; i < pml0; ++i) {
+        BlendCoef c;
+        blend_coef_init(c, i, pml0);
+        for (long long t = 0; t < trials; ++t) {
+            const int e = E(rng);
+            float q = (float)std::ldexp(U(rng), e), a = (float)(q * (1.0 + 0.3 * U(rng)) * c.w);
+            switch (t % 8) {
+            case 1: a = (float)std::ldexp(U(rng), E(rng)); break;
+            case 2: a = (float)(-c.omw * q * (1.0 + std::ldexp(U(rng), -(int)(t / 8 % 30)))); break;
+            case 3: q = std::ldexp((float)M(rng), e / 2); a = std::ldexp((float)M(rng), e / 2 - 1); break;
+            case 4:
+            case 5: {
+                const float target = (float)(4.0 * U(rng));
+                if (c.omw > 0) q = (float)((0.5 * ((double)target + std::nextafter(target, 9.0f)) - a) / c.omw);
+                break;
+            }
+            case 6: (t & 8 ? a : q) = t & 16 ? INFINITY : -INFINITY; break;
+            case 7: if (t & 8) q = t & 16 ? 0.0f : -0.0f; break;
+            default: break;
+            }
+            const float got = blend_mix_values(a, q, c.bh, c.bl, c.khi2, c.klo2, fp32_ok);
+            const float want = (float)((double)a + c.omw * (double)q);
+            bad += !same(got, want) && !(std::isnan(got) && std::isnan(want));
+        }
+    }
+    return bad;
+}
+
 }  // extern "C"

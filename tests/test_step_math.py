@@ -22,6 +22,7 @@ def harness(tmp_path_factory):
     L.harness_quotients_at_their_bounds.argtypes, L.harness_quotients_at_their_bounds.restype = [f], ll
     L.harness_div2_least.argtypes, L.harness_div2_least.restype = [f], f
     L.harness_mix.argtypes, L.harness_mix.restype = [i, ll, ctypes.c_uint, ctypes.POINTER(ll)], ll
+    L.harness_mix_values.argtypes, L.harness_mix_values.restype = [i, ll, ctypes.c_uint, i], ll
     return L
 
 
@@ -72,3 +73,8 @@ def test_tails_of_divisors_of_many_bits(harness, y):
 
 def test_divisors_whose_low_word_leaves_no_room_for_tails_are_refused(harness):
     assert harness.harness_two_op_exact(2500.3) == 1 and harness.harness_quotients_at_their_bounds(2500.3) == -1
+
+
+@pytest.mark.parametrize("pml0", [1, 2, 8, 10, 13, 20, 40, 77, 300])  # from 33 on, some 1 - w have over 29 bits
+def test_mix_by_value_matches_the_double_formula(harness, pml0):
+    assert harness.harness_mix_values(pml0, max(4000, 640000 // pml0), 9 + pml0, 1 if pml0 <= 32 else 0) == 0
