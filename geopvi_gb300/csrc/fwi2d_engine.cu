@@ -412,7 +412,9 @@ static Layout plan_layout(const Geom &g, int nsamples, int resident, bool syn_in
 
 // Padded v*dt for every sample: get_velp's replication (a clamp) times dt,
 // the float product that powf(v*dt, 2) and s = v*dt/dx start from.
-// status[1] is set where a velocity's (v dt)^2 is not finite.
+// status[1] is set where a velocity's (v dt)^2, or a product of abc_for_p's
+// factors of s = v dt / dx, may not be finite (s above 10^4; a stable scheme's is
+// below 1).
 __global__ void k_prepare(const Geom g, const float *__restrict__ vel, float *__restrict__ vdt, int nsamples,
                           int *__restrict__ status)
 {
@@ -426,7 +428,7 @@ __global__ void k_prepare(const Geom g, const float *__restrict__ vel, float *__
         float v = 0.0f;
         if (ix >= 0 && ix < g.ntx)
             v = fm(padded_velocity(g, vel + (long long)s * g.nx * g.nz, iz, ix), g.dt);
-        if (!isfinite(fm(v, v))) atomicOr(status + 1, 1);
+        if (!isfinite(fm(v, v)) || fabsf(v) > 1e4f * g.dx) atomicOr(status + 1, 1);
         vdt[e] = v;
     }
 }

@@ -588,8 +588,7 @@ __device__ __forceinline__ bool tile_is_zero(const float *tile, int n4, int mid,
     return !__any_sync(kAll, (bits & 0x7fffffffu) != 0u);
 }
 
-// The new level of such a tile, and its stored field (interior tiles; the
-// adjoint's terms add nothing).
+// The new level of such a tile, and its stored field (interior tiles).
 __device__ __forceinline__ void zero_tile(const Geom &g, const WarpCtx &w, int nrows, bool wide, bool interior)
 {
     float *p2 = w.p2 + w.lane, *ps = w.ps + w.lane;
@@ -604,6 +603,26 @@ __device__ __forceinline__ void zero_tile(const Geom &g, const WarpCtx &w, int n
         }
         p2 += w.st;
         ps += w.si;
+    }
+}
+
+// The adjoint's terms of such a tile, rows of columns c0, c0 + 32, .. < c1: zeros,
+// but NaN where a stored value is not finite (a forward pass that overflowed).
+// s0, s1, s2: null where there is none.  Out of line, so its registers are not the
+// sweeps' (inlined, order 8 spilled 20 bytes).  Reading the stored field here
+// takes 0.6 % of 80 solves of 200x400; a look at the last forward level instead
+// costs the forward kernel spills, 1.5 %.
+static __device__ __noinline__ void zero_terms(const float *s0, const float *s1, const float *s2, float *G, int si,
+                                               int nrows, int c0, int c1)
+{
+    for (int j = 0; j < nrows; ++j) {
+        const int o = j * si;
+        for (int c = c0; c < c1; c += 32) {
+            float t = s0 ? fm(__ldcs(s0 + o + c), 0.0f) : 0.0f;
+            if (s1) t = ff(__ldcs(s1 + o + c), 0.0f, t);
+            if (s2) t = ff(__ldcs(s2 + o + c), 0.0f, t);
+            if (!(t == 0.0f)) G[o + c] = t;
+        }
     }
 }
 
