@@ -657,6 +657,15 @@ static int step_variant_for(const Geom &g, long long nres)
     return nres * step_tiles(g, 4) >= 5000 ? 2 : 3;
 }
 
+// A forced variant, or taller tiles where a solve has more of them than a grid's y
+// extent holds (the values are the same; step_variant_for's choices never do,
+// short of 33 M cells).
+static int fit_variant(const Geom &g, int variant)
+{
+    while (variant > 0 && step_tiles(g, kStepVariants[variant].rows) > 65535) --variant;
+    return variant;
+}
+
 // ---------------------------------------------------------------------------
 // Pseudo-spectral mode: cuFFT, loaded on first use (the FD path needs no
 // FFT library), batched 2-D Z2Z plans cached per (device, grid, batch).
@@ -1885,7 +1894,7 @@ static int batch_impl(const gb_fwi2d_params *p, int nsamples, const float *vel, 
     c.clear_status = clear_status;
     const unsigned forced = (flags >> GB_FWI2D_VARIANT_SHIFT) & 0xFu;
     if (forced > (unsigned)kNumStepVariants) return GB_FWI2D_EINVAL;
-    c.variant = forced ? (int)forced - 1 : step_variant_for(d.g, (flags & GB_FWI2D_PLAIN) ? 1 : L.resident);
+    c.variant = forced ? fit_variant(d.g, (int)forced - 1) : step_variant_for(d.g, (flags & GB_FWI2D_PLAIN) ? 1 : L.resident);
     if (!make_call_maps(c, d.g, L, flags)) return GB_FWI2D_ECUDA;
     st = get_tables(d, c.tab);
     if (st) return st;

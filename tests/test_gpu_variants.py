@@ -76,3 +76,16 @@ def test_tuner_tries_a_variant_per_wave(engine_lib, cuda):
     assert np.array_equal(g0, g1)
     ref = Fwi2dEngine(p, device="cuda:0", graph=False, variant=0).run(v, o).grad.cpu().numpy()
     assert np.array_equal(g0, ref)
+
+
+def test_forced_variant_on_a_grid_of_many_tiles(engine_lib, cuda):
+    """More two-row tiles in a solve than a grid's y extent holds: the values come from taller ones."""
+    from geopvi_gb300.engine import Fwi2dEngine
+    from geopvi_gb300.params import Params
+    p = Params(nx=30000, nz=300, pml0=5, Lc=4, ns=1, nt=12, ds=1, ns0=15000, depths=2, depthr=0, nr=3000, dr=1, nr0=13500,
+               nt_interval=1, dx=10.0, dz=10.0, dt=1e-3, f0=60.0)
+    v = torch.full((1, p.nz * p.nx), 2500.0, device=cuda)
+    o = torch.zeros(p.data_len, device=cuda)
+    want = Fwi2dEngine(p, device=cuda).run(v, o, forward_only=True).syn
+    got = Fwi2dEngine(p, device=cuda, variant=3).run(v, o, forward_only=True).syn
+    assert want.abs().max() > 0 and torch.equal(got, want)
