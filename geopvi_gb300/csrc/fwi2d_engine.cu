@@ -596,17 +596,22 @@ static bool make_map(CUtensorMap &m, void *base, const Geom &g, long long depth,
 static thread_local int t_enqueue_error = 0;
 
 static std::mutex g_side_mutex;
-static std::map<std::pair<int, std::thread::id>, SideStream> g_side;
+struct SideStreams {
+    SideStream of[kMaxSideStreams];
+    int n = 0;
+};
+static std::map<std::pair<int, std::thread::id>, SideStreams> g_side;
 
-const SideStream *side_stream(bool create)
+const SideStream *side_stream(cudaStream_t caller, bool create)
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     std::lock_guard<std::mutex> lk(g_side_mutex);
-    const auto key = std::make_pair(dev, std::this_thread::get_id());
-    auto it = g_side.find(key);
-    if (it != g_side.end()) return &it->second;
-    if (!create) return nullptr;
+    SideStreams &mine = g_side[std::make_pair(dev, std::this_thread::get_id())];
+    for (int i = 0; i < mine.n; ++i)
+        if (mine.of[i].caller == caller) return &mine.of[i];
+    if (mine.n == kMaxSideStreams) return &mine.of[((uintptr_t)caller >> 4) % kMaxSideStreams];
+    if (!create) return mine.n ? &mine.of[0] : nullptr;
     SideStream ss;
     if (cudaStreamCreateWithFlags(&ss.s, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
     if (cudaEventCreateWithFlags(&ss.fork, cudaEventDisableTiming) != cudaSuccess ||
@@ -615,7 +620,8 @@ const SideStream *side_stream(bool create)
         cudaStreamDestroy(ss.s);
         return nullptr;
     }
-    return &(g_side[key] = ss);
+    ss.caller = caller;
+    return &(mine.of[mine.n++] = ss);
 }
 
 // Waves of at least this many resident solves, or two whose launches have this
@@ -1056,7 +1062,7 @@ static long long enqueue_exact(const Call &c, cudaStream_t st)
     cudaStreamIsCapturing(st, &cs);
     const SideStream *side = (!split_wave(wave, tiles) || c.single_stream)
                                  ? nullptr
-                                 : side_stream(cs == cudaStreamCaptureStatusNone);
+                                 : side_stream(st, cs == cudaStreamCaptureStatusNone);
     // The steps leave the rim of the levels they write as it is: zero, once
     // for all waves (later writes to a level never touch its rim).
     cudaMemsetAsync(store, 0, store_pitch * std::min<long long>(wave, ninst), st);
@@ -1192,7 +1198,7 @@ static long long enqueue(const Call &c, cudaStream_t st)
     const int tiles = g.pstd ? 0 : step_tiles(g, kStepVariants[c.variant].rows);
     const SideStream *side = (g.pstd || !split_wave(wave, tiles) || c.single_stream)
                                  ? nullptr
-                                 : side_stream(cs == cudaStreamCaptureStatusNone);
+                                 : side_stream(st, cs == cudaStreamCaptureStatusNone);
     const bool ckpt = (c.flags & GB_FWI2D_CHECKPOINT) && !fwd_only;
     for (long long i0 = 0; i0 < ninst && ckpt; i0 += wave) {
         const int nres = (int)std::min<long long>(wave, ninst - i0);
@@ -1506,7 +1512,7 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
     int *status = (int *)work;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(st, &cs);
-    const SideStream *side = side_stream(cs == cudaStreamCaptureStatusNone);
+    const SideStream *side = side_stream(st, cs == cudaStreamCaptureStatusNone);
     size_t off = kFusedHeader;
     for (auto &f : fi) {
         f.rik = off;
@@ -1774,7 +1780,7 @@ static int run_graph(const Call &c, cudaStream_t st, long long &launches)
                                                                       : GB_FWI2D_ECUDA;
         }
     }
-    side_stream(true);  // created outside the capture
+    side_stream(st, true);  // created outside the capture
     cudaStream_t cap;
     if (cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess) return GB_FWI2D_ECUDA;
     cudaGraph_t graph = nullptr;
@@ -2087,7 +2093,9 @@ double gb_fwi2d_profile_step_ms(long long *launches)
 int gb_fwi2d_side_stream_count(void)
 {
     std::lock_guard<std::mutex> lk(g_side_mutex);
-    return (int)g_side.size();
+    int n = 0;
+    for (const auto &kv : g_side) n += kv.second.n;
+    return n;
 }
 
 void gb_fwi2d_release_caches(void)
@@ -2106,11 +2114,12 @@ void gb_fwi2d_release_caches(void)
     for (auto &kv : g_kk_tables) cudaFree(kv.second);
     g_kk_tables.clear();
     std::lock_guard<std::mutex> lk2(g_side_mutex);
-    for (auto &kv : g_side) {
-        cudaEventDestroy(kv.second.fork);
-        cudaEventDestroy(kv.second.join);
-        cudaStreamDestroy(kv.second.s);
-    }
+    for (auto &kv : g_side)
+        for (int i = 0; i < kv.second.n; ++i) {
+            cudaEventDestroy(kv.second.of[i].fork);
+            cudaEventDestroy(kv.second.of[i].join);
+            cudaStreamDestroy(kv.second.of[i].s);
+        }
     g_side.clear();
 }
 

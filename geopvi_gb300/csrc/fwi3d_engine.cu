@@ -1084,7 +1084,7 @@ int gb_fwi3d_run(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int nsamples, 
     const int inject_blocks = std::min(64, (g.nu + io_threads - 1) / io_threads);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(st, &cs);
-    const SideStream *side = split_wave(g, L.resident) ? side_stream(cs == cudaStreamCaptureStatusNone) : nullptr;
+    const SideStream *side = split_wave(g, L.resident) ? side_stream(st, cs == cudaStreamCaptureStatusNone) : nullptr;
     for (long long i0 = 0; i0 < ninst; i0 += L.resident) {
         const int nres = (int)std::min<long long>(L.resident, ninst - i0);
         b.inst0 = ba.inst0 = (int)i0;

@@ -6,17 +6,23 @@
 
 namespace gbfwi {
 
-// The schedule's second stream, per (device, host thread), with its fork / join
-// events.  Kept for the process (a graph capture records work on it) and freed
-// by gb_fwi2d_release_caches.
+// The schedule's second stream, per (device, host thread, caller's stream), with
+// its fork / join events.  Kept for the process (a graph capture records work on
+// it) and freed by gb_fwi2d_release_caches.
 struct SideStream {
     cudaStream_t s = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
+    cudaStream_t caller = nullptr;
 };
 
-// This thread's side stream on the current device; created on first use
-// unless `create` is false (a stream being captured by the caller).
-const SideStream *side_stream(bool create);
+// A thread has at most this many on a device; callers' streams beyond share them.
+constexpr int kMaxSideStreams = 8;
+
+// The side stream of this thread's work on `caller`, on the current device: its
+// own, so that calls on different streams do not queue behind one another.
+// Created on first use unless `create` is false (a stream being captured), which
+// takes any that the thread has: a capture records on it and queues nothing.
+const SideStream *side_stream(cudaStream_t caller, bool create);
 
 // A wave's two halves (or, without a side stream, the whole wave): the solves
 // [0, nlo) on st and [nlo, nres) on the side stream, between fork() and join().
