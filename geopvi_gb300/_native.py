@@ -56,6 +56,7 @@ EXPORTED_SYMBOLS = (
     "gb_fwi2d_release_caches", "gb_fwi2d_version", "gb_fwi2d_profile_step_ms", "gb_fwi2d_status",
     "gb_fwi2d_batch_noalloc", "gb_fwi2d_tuned_variant", "gb_fwi2d_instances_workspace_bytes",
     "gb_fwi2d_run_instances", "gb_fwi2d_side_stream_count", "gb_fwi2d_instances_waves",
+    "gb_fwi2d_graph_launches",
 )
 
 
@@ -131,6 +132,8 @@ def load() -> ctypes.CDLL:
         L.gb_fwi2d_instances_waves.restype = ctypes.c_int
         L.gb_fwi2d_side_stream_count.argtypes = []
         L.gb_fwi2d_side_stream_count.restype = ctypes.c_int
+        L.gb_fwi2d_graph_launches.argtypes = []
+        L.gb_fwi2d_graph_launches.restype = ctypes.c_longlong
         L.gb_fwi2d_release_caches.argtypes = []
         L.gb_fwi2d_release_caches.restype = None
         L.gb_fwi2d_version.argtypes = []

@@ -526,11 +526,17 @@ struct DeviceTables {
 struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
     long long launches = 0;
+    long long used = 0;  // the call that last launched it, by g_graph_calls
 };
+// A graph belongs to its call's buffers, and a pass is up to tens of thousands of
+// launches: a program whose buffers move keeps the graphs it used last, with at
+// most this many launches in all (7.5 KB of host and 2.6 KB of device memory each).
+constexpr long long kMaxGraphLaunches = 1 << 18;
 
 static std::mutex g_mutex;
 static std::map<std::pair<int, int>, DeviceTables> g_tables;  // (device, pml0)
 static std::map<std::vector<long long>, GraphEntry> g_graphs;
+static long long g_graph_calls = 0;
 static thread_local long long t_last_launches = 0;
 
 // Event pairs around the step-kernel loops of profiled calls, accumulated
@@ -1776,6 +1782,7 @@ static int run_graph(const Call &c, cudaStream_t st, long long &launches)
         auto it = g_graphs.find(key);
         if (it != g_graphs.end()) {
             launches = it->second.launches;
+            it->second.used = ++g_graph_calls;
             return cudaGraphLaunch(it->second.exec, st) == cudaSuccess ? GB_FWI2D_OK
                                                                       : GB_FWI2D_ECUDA;
         }
@@ -1796,12 +1803,23 @@ static int run_graph(const Call &c, cudaStream_t st, long long &launches)
     e = cudaGraphInstantiate(&ge.exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return GB_FWI2D_ECUDA;
-    ge.launches = n;
-    {
-        std::lock_guard<std::mutex> lk(g_mutex);
-        g_graphs[key] = ge;
+    ge.launches = launches = n;
+    std::lock_guard<std::mutex> lk(g_mutex);
+    GraphEntry &kept = g_graphs[key];
+    if (kept.exec) cudaGraphExecDestroy(kept.exec);  // another thread captured the same call meanwhile
+    kept = ge;
+    kept.used = ++g_graph_calls;
+    for (;;) {  // a graph in flight is freed when it completes
+        long long total = 0;
+        auto oldest = g_graphs.begin();
+        for (auto it = g_graphs.begin(); it != g_graphs.end(); ++it) {
+            total += it->second.launches;
+            if (it->second.used < oldest->second.used) oldest = it;
+        }
+        if (total <= kMaxGraphLaunches || g_graphs.size() == 1) break;
+        cudaGraphExecDestroy(oldest->second.exec);
+        g_graphs.erase(oldest);
     }
-    launches = n;
     return cudaGraphLaunch(ge.exec, st) == cudaSuccess ? GB_FWI2D_OK : GB_FWI2D_ECUDA;
 }
 
@@ -2095,6 +2113,14 @@ int gb_fwi2d_side_stream_count(void)
     std::lock_guard<std::mutex> lk(g_side_mutex);
     int n = 0;
     for (const auto &kv : g_side) n += kv.second.n;
+    return n;
+}
+
+long long gb_fwi2d_graph_launches(void)
+{
+    std::lock_guard<std::mutex> lk(g_mutex);
+    long long n = 0;
+    for (const auto &kv : g_graphs) n += kv.second.launches;
     return n;
 }
 

@@ -215,9 +215,15 @@ int gb_fwi2d_batch_noalloc(const gb_fwi2d_params *p, int nsamples, const float *
 int gb_fwi2d_status(const void *work, void *stream);
 
 /* Diagnostic: the number of auxiliary CUDA streams the library holds (one
- * per device and host thread that ran gb_fwi2d_batch's two-stream schedule;
- * released by gb_fwi2d_release_caches).  No counterpart in the reference. */
+ * per device, host thread and caller's stream that ran the two-stream schedule,
+ * at most 8 a thread; released by gb_fwi2d_release_caches).  No counterpart in
+ * the reference. */
 int gb_fwi2d_side_stream_count(void);
+
+/* Diagnostic: the kernel launches in the CUDA graphs that the library keeps
+ * (GB_FWI2D_GRAPH; the graphs used last, 262144 launches at most).  No
+ * counterpart in the reference. */
+long long gb_fwi2d_graph_launches(void);
 
 /* Number of kernel launches the last gb_fwi2d_batch call on this thread
  * enqueued (graph replays count the kernels inside the graph). */
