@@ -414,11 +414,13 @@ static Layout plan_layout(const Geom &g, int nsamples, int resident, bool syn_in
 // the float product that powf(v*dt, 2) and s = v*dt/dx start from.
 // status[1] is set where a velocity's (v dt)^2, or a product of abc_for_p's
 // factors of s = v dt / dx, may not be finite (s above 10^4; a stable scheme's is
-// below 1).
+// below 1), and for a grid with tiles on the rim, which have no field around them
+// to look at.
 __global__ void k_prepare(const Geom g, const float *__restrict__ vel, float *__restrict__ vdt, int nsamples,
                           int *__restrict__ status)
 {
     const long long total = (long long)nsamples * g.fstride;
+    if (g.tile_r0 == 0 && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(status + 1, 2);
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
         const int s = (int)(e / g.fstride);

@@ -99,7 +99,7 @@ struct Batch {
     float *gacc;         // [nsamples*ns][pstride]
     const BlendCoef *coef;  // [pml0] boundary weight w, 1 - w split in floats and as double
     int blend_fp32;      // the host proved (1 - w) * q exact in double for every weight
-    int *status;         // device error word (0 = ok), then k_prepare's flag
+    int *status;         // device error word (0 = ok), then k_prepare's flags
     int inst0;           // first solve of this wave
     int slot0;           // first resident slot of this launch (the wave's second half)
     int levels;          // fields per resident slot of `ring`: 3, or the levels of a stored segment
@@ -157,7 +157,7 @@ __host__ __device__ __forceinline__ StepArgs ring_step(int k, int it, int snap, 
 }
 
 enum : int { kStatusOk = 0, kStatusTmaTimeout = 1 };
-constexpr int kStatusWords = 2;  // the error word, and k_prepare's flag of non-finite velocities
+constexpr int kStatusWords = 2;  // the error word, and k_prepare's flags: no tile is skipped
 
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }

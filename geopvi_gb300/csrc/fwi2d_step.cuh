@@ -570,14 +570,15 @@ __device__ __forceinline__ bool tile_is_zero(const float *tile, int n4, int mid,
 {
     constexpr unsigned kAll = 0xffffffffu;
     if (__any_sync(kAll, tile[mid + w.lane] != 0.0f)) return false;
-    unsigned bits = (unsigned)status[1];
+    unsigned bits = (unsigned)status[1];  // flagged: returns before p0 is read
     for (int i = w.lane; i < n4; i += 32) {
         const uint4 v = reinterpret_cast<const uint4 *>(tile)[i];
         bits |= (v.x | v.y | v.z | v.w) & 0x7fffffffu;
     }
     if (__any_sync(kAll, bits != 0u)) return false;
     // The blends read p0 up to 4 rows and columns inward; tiles lie at least
-    // that far inside the field's memory, row padding included.
+    // that far inside the field's memory, row padding included, but for grids with
+    // tiles on the rim, where k_prepare's flag leaves none to look at.
     const float *p0 = w.p0 + w.lane;
     if (wide) {
         for (int j = 0; j < nrows; ++j, p0 += w.st) bits |= __float_as_uint(p0[0]) | __float_as_uint(p0[32]);

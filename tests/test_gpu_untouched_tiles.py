@@ -77,3 +77,16 @@ def test_overflow_in_one_inversion_of_a_fused_call(engine_lib, cuda, oracle):
     _native.check(st, "gb_fwi2d_run_instances")
     for _, _, _, g, ref in parts:
         assert np.array_equal(np.isfinite(g[0].cpu().numpy()), np.isfinite(ref))
+
+
+@pytest.mark.parametrize("change,flag", [(dict(), 0), (dict(depthr=-12), 2), (dict(nr=176, nr0=-13), 2)])
+def test_tiles_on_the_rim_are_not_looked_at(engine_lib, cuda, oracle, change, flag):
+    """A tile at the end of a field's rows has no memory of the field beside it to look at: none is skipped then."""
+    from geopvi_gb300.engine import Fwi2dEngine
+    p = Params(**{**BASE, "depths": 2, **change})
+    vel = np.full((p.nz, p.nx), 2000.0, np.float32)
+    obs = np.zeros(p.data_len, np.float32)
+    eng = Fwi2dEngine(p, device=cuda)
+    r = eng.run(torch.from_numpy(vel.ravel()).to(cuda)[None], torch.from_numpy(obs).to(cuda), forward_only=True)
+    assert int(eng._work[4:8].view(torch.int32)) == flag
+    assert np.array_equal(r.syn[0].cpu().numpy(), solve(oracle, p, vel, obs)[0])
