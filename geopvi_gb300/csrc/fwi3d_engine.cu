@@ -843,6 +843,11 @@ static Layout3 plan(const Geom3 &g, int nsamples, int resident, bool fwd_only, b
     return L;
 }
 
+// A workspace may start anywhere: the layout does at its first multiple of
+// kWorkAlign (the tensor maps need 16 bytes), for which its size has room.
+constexpr size_t kWorkAlign = 256;
+static size_t work_bytes_of(const Layout3 &L) { return L.total + kWorkAlign; }
+
 static thread_local long long t_launches = 0;
 
 static int grid_for(long long n, int block)
@@ -992,9 +997,8 @@ int gb_fwi3d_workspace_size(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int
     if (st) return st;
     Host3 h;
     derive(*p, *a, h);
-    *bytes = plan(h.g, nsamples, max_resident, (flags & GB_FWI3D_FORWARD_ONLY) != 0,
-                  (flags & GB_FWI3D_CHECKPOINT) != 0, true)
-                 .total;
+    *bytes = work_bytes_of(plan(h.g, nsamples, max_resident, (flags & GB_FWI3D_FORWARD_ONLY) != 0,
+                                (flags & GB_FWI3D_CHECKPOINT) != 0, true));
     return GB_FWI2D_OK;
 }
 
@@ -1008,7 +1012,7 @@ int gb_fwi3d_max_resident(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int n
     long long lo = 0, hi = std::min<long long>((long long)nsamples * p->ns, 65535);
     while (lo < hi) {
         const long long mid = (lo + hi + 1) / 2;
-        if (plan(h.g, nsamples, (int)mid, fo, ck, true).total <= budget)
+        if (work_bytes_of(plan(h.g, nsamples, (int)mid, fo, ck, true)) <= budget)
             lo = mid;
         else
             hi = mid - 1;
@@ -1034,9 +1038,9 @@ int gb_fwi3d_run(const gb_fwi3d_params *p, const gb_fwi3d_acq *a, int nsamples, 
     derive(*p, *a, h);
     const Geom3 &g = h.g;
     const Layout3 L = plan(g, nsamples, max_resident, fwd_only, ckpt, syn == nullptr);
-    if (L.total > work_bytes) return GB_FWI2D_ENOMEM;
+    char *w = (char *)a256((size_t)work);
+    if (L.total + (size_t)(w - (char *)work) > work_bytes) return GB_FWI2D_ENOMEM;
     cudaStream_t st = (cudaStream_t)stream;
-    char *w = (char *)work;
     Maps3 tm, tm_adj;
     auto maps = [&](Maps3 &m, size_t ring) { return make_maps3(m, w + ring, 3LL * L.resident, w + L.vdt, nsamples, g); };
     if (!prepare_device(g.L - 1) || !maps(tm, L.ring)) return GB_FWI2D_ECUDA;

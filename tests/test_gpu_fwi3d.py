@@ -199,3 +199,25 @@ def test_a_wait_that_gave_up_leaves_no_data(engine_lib, cuda):
     torch.cuda.synchronize()
     assert torch.isnan(r.syn).all() and torch.isnan(r.misfit).all()
     assert torch.equal(eng.run(vel, small, forward_only=True).syn, good)
+
+
+@pytest.mark.parametrize("offset", [4, 8, 200])
+def test_workspace_at_any_address(engine_lib, cuda, offset):
+    import ctypes
+    from geopvi_gb300 import _native, workloads
+    p = fwi3d.Fwi3dParams(nx=30, ny=21, nz=17, nt=40, dt=1e-3, pml0=6, Lc=4)
+    rec = np.array([[x, 10, 0] for x in range(0, 30, 3)])
+    eng = fwi3d.Fwi3dEngine(p, np.array([[8, 9, 2]]), rec, workloads.ricker(p.nt, p.dt, 25.0), device=cuda)
+    vel = torch.full((1, p.ncell), 2300.0, device=cuda)
+    obs = 0.01 * torch.randn(p.nt * len(rec), device=cuda)
+    want = eng.run(vel, obs, want_syn=True)
+    nbytes = eng.workspace_bytes(1, 1)
+    room = torch.zeros(nbytes + 256, dtype=torch.uint8, device=cuda)
+    syn, grad = torch.empty_like(want.syn), torch.empty_like(want.grad)
+    st = eng.lib.gb_fwi3d_run(ctypes.byref(eng.cp), ctypes.byref(eng.acq.c), 1, ctypes.c_void_p(vel.data_ptr()),
+                              ctypes.c_void_p(obs.data_ptr()), ctypes.c_void_p(syn.data_ptr()),
+                              ctypes.c_void_p(grad.data_ptr()), None, ctypes.c_void_p(room.data_ptr() + offset), nbytes, 1,
+                              0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    _native.check(st, "gb_fwi3d_run")
+    assert torch.equal(syn, want.syn) and torch.equal(grad, want.grad)
+    assert not room[:offset].any() and not room[nbytes + offset:].any()
