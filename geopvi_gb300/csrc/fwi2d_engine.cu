@@ -1567,7 +1567,7 @@ static long long run_fused_chunk(std::vector<FusedInst> &fi, std::vector<FusedWa
         auto seconds = [&](const FusedLaunch &l) {
             double cells = 0.0;
             for (int j : l.pieces) cells += (double)w.pieces[j].r * fi[w.pieces[j].inst].d.g.fstride;
-            return l.maxnt * (6e-6 + 4e-12 * cells);
+            return l.maxnt * (6e-6 + 4e-12 * cells);  // only compared with one another
         };
         double total = 0.0, load[2] = {0.0, 0.0};
         for (const auto &l : w.launches) total += seconds(l);

@@ -42,9 +42,13 @@ from .params import Params
 # (f = 0.07: 1000x2000, 8 solves, 218 G cell-updates/s; f = 0.29: 200x400,
 # 200 solves, 166 G; f = 0.91: 16x32, 4000 solves, 85 G), within 7 % of each;
 # the fixed cost is the latency of one small launch (one 200x400 solve per
-# step: ~22 us).  Fitted to the one-column step kernel; the present one takes
-# about two thirds of these times and a quarter of the fixed cost.  Plans compare
-# times, so their choice depends on the ratios only.
+# step: ~22 us).  Fitted to the one-column step kernel.  The same fit of the
+# present one (11 sizes from 32x48 to 1000x2000, 2 to 4000 solves, within 18 %)
+# gives 1.93e-12, 6.86e-12 and 4.2e-6: the fixed cost has fallen 2.6 times as far
+# as the cells', so these constants overrate small waves' launches.  They stay
+# because they decide between storage modes and calls (with the new ones, 32
+# models of 400x800 x 40 shots in 75 GB would be stored whole in waves of 8
+# instead of checkpointed in waves of 179), and those choices are not measured.
 CELL_S = 3.78e-12
 STRIP_CELL_S = 8.69e-12
 LAUNCH_OVERHEAD_S = 20e-6
