@@ -44,8 +44,8 @@ from .params import Params
 # the fixed cost is the latency of one small launch (one 200x400 solve per
 # step: ~22 us).  Fitted to the one-column step kernel.  The same fit of the
 # present one (11 sizes from 32x48 to 1000x2000, 2 to 4000 solves, within 18 %)
-# gives 1.93e-12, 6.86e-12 and 4.2e-6: the fixed cost has fallen 2.6 times as far
-# as the cells', so these constants overrate small waves' launches.  They stay
+# gives 1.93e-12, 6.86e-12 and 4.2e-6: the fixed cost has fallen 2.5 to 4 times as
+# far as the cells', so these constants overrate small waves' launches.  They stay
 # because they decide between storage modes and calls (with the new ones, 32
 # models of 400x800 x 40 shots in 75 GB would be stored whole in waves of 8
 # instead of checkpointed in waves of 179), and those choices are not measured.

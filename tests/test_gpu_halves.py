@@ -72,3 +72,26 @@ def test_exact_gradient_halves_match_single_solves(engine_lib, cuda, nz, nx, ns,
     ref = Fwi2dEngine(p, device=cuda, graph=False, max_resident=1).run(vel, obs, exact=True)
     r = Fwi2dEngine(p, device=cuda, **kw).run(vel, obs, exact=True)
     assert torch.equal(r.grad, ref.grad) and torch.equal(r.misfit, ref.misfit)
+
+
+@pytest.mark.parametrize("kw", (dict(), dict(checkpoint=True)))
+@pytest.mark.parametrize("ns,nsamples", ((7, 2), (5, 3)))  # waves of 5, 5 and 4 solves (4 are below the line), of 5, 5, 5
+def test_halves_3d_over_several_waves(engine_lib, cuda, ns, nsamples, kw):
+    """Five of these solves (2 x 5 tiles, 80 planes each: 4000) run as halves of two and three, wave after wave."""
+    import numpy as np
+    import torch
+    from geopvi_gb300 import fwi3d
+    rng = np.random.default_rng(6)
+    nx, ny, nz, nt = 70, 61, 64, 26
+    p = fwi3d.Fwi3dParams(nx=nx, ny=ny, nz=nz, nt=nt, dt=1e-3, dx=10.0, dy=10.0, dz=10.0, pml0=8, Lc=4)
+    src = np.stack([rng.integers(20, 45, ns) for _ in range(3)], 1).astype(np.int32)
+    rec = np.stack([rng.integers(0, m, 40) for m in (nx, ny, nz)], 1).astype(np.int32)
+    wavelet = rng.standard_normal(nt).astype(np.float32)
+    vel = torch.from_numpy((2500 + 200 * rng.standard_normal((nsamples, nx * ny * nz))).astype(np.float32)).to(cuda)
+    obs = torch.from_numpy(rng.standard_normal(ns * nt * len(rec)).astype(np.float32)).to(cuda)
+    ref = fwi3d.Fwi3dEngine(p, src, rec, wavelet, device=cuda, max_resident=1, **kw).run(vel, obs, want_syn=True)
+    eng = fwi3d.Fwi3dEngine(p, src, rec, wavelet, device=cuda, max_resident=5, **kw)
+    assert eng.resident_for(nsamples) == 5
+    r = eng.run(vel, obs, want_syn=True)
+    for name in ("syn", "grad", "misfit"):
+        assert torch.equal(getattr(r, name), getattr(ref, name)), name

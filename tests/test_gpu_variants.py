@@ -89,3 +89,23 @@ def test_forced_variant_on_a_grid_of_many_tiles(engine_lib, cuda):
     want = Fwi2dEngine(p, device=cuda).run(v, o, forward_only=True).syn
     got = Fwi2dEngine(p, device=cuda, variant=3).run(v, o, forward_only=True).syn
     assert want.abs().max() > 0 and torch.equal(got, want)
+
+
+# Sizes around each line of the rule: samples and shots of a grid, the variant (rows 16, 8, 4, 2).
+@pytest.mark.parametrize("nz,nx,ns,n,variant", [
+    (32, 48, 2, 1, 3), (120, 250, 16, 1, 3), (120, 250, 16, 2, 2), (120, 250, 16, 3, 1), (120, 250, 16, 9, 1),
+    (120, 250, 16, 10, 0), (200, 400, 20, 4, 1), (200, 400, 20, 5, 0),
+])
+def test_rule_of_the_tile_height(engine_lib, cuda, nz, nx, ns, n, variant):
+    from geopvi_gb300 import workloads
+    from geopvi_gb300.engine import Fwi2dEngine
+    p = workloads.make_params(nz, nx, 20, 1e-3, ns, 30.0, pml0=20)
+    g = torch.Generator(device=cuda).manual_seed(3)
+    v = (2500 + 200 * torch.randn(n, nz * nx, generator=g, device=cuda)).clamp(1500, 4500)
+    o = 0.01 * torch.randn(p.data_len, generator=g, device=cuda)
+    eng = Fwi2dEngine(p, device=cuda)
+    r = eng.run(v, o, want_syn=True)
+    assert eng.tuned_variant(n) == variant
+    other = Fwi2dEngine(p, device=cuda, variant=(variant + 1) % 4).run(v, o, want_syn=True)
+    for name in ("syn", "grad", "misfit"):
+        assert torch.equal(getattr(r, name), getattr(other, name)), name
