@@ -87,11 +87,17 @@ def cell_updates_per_sample(p) -> int:
     return 2 * p.ns * p.nt * p.ntp
 
 
+def imaging_bytes(p) -> int:
+    """Per shot: 4 B written and 4 B read of every interior cell of a stored
+    step, and a read and write of the accumulator every third step (or stored
+    step, where those are fewer)."""
+    return 8 * (p.nt_save + min(p.nt_save, -(-p.nt // 3))) * p.ncell
+
+
 def algorithmic_bytes_per_sample(p) -> int:
-    """16 B per propagation cell-update (read p0, p1, v*dt; write p2) plus,
-    per interior cell per stored step, 4 B written forward and 12 B in the
-    adjoint (read the stored field, read-modify-write the accumulator)."""
-    return p.ns * (2 * p.nt * 16 * p.ntp + p.nt_save * 16 * p.ncell)
+    """16 B per propagation cell-update (read p0, p1, v*dt; write p2), and the
+    imaging."""
+    return p.ns * (2 * p.nt * 16 * p.ntp + imaging_bytes(p))
 
 
 # ---------------------------------------------------------------------------
@@ -519,7 +525,7 @@ def run_autograd(args):
     cu_batch = cell_updates_per_sample(p) * nsamples
     value = args.steps * cu_batch / (ms / 1e3)
     # roofline of the step kernel over every launched step (forward, recomputed forward, adjoint)
-    alg = nsamples * p.ns * (3 * p.nt * 16 * p.ntp + p.nt_save * 16 * p.ncell) * args.steps
+    alg = nsamples * p.ns * (3 * p.nt * 16 * p.ntp + imaging_bytes(p)) * args.steps
     peak, peak_src = peak_hbm()
     achieved = alg / (step_ms / 1e3) / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,

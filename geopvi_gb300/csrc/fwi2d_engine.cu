@@ -1389,8 +1389,8 @@ static size_t fused_min_bytes(const FusedInst &f, bool fwd_only)
 }
 
 // Flags under which gb_fwi2d_run_instances fuses instances (full storage,
-// the reference's gradient, launches enqueued directly; the fused kernel has
-// one variant, so a forced variant does not apply to it).
+// the reference's gradient, launches enqueued directly; each fused launch takes
+// the variant that step_variant_for gives it, a forced one does not apply).
 static bool fusable(unsigned flags)
 {
     return !(flags & (GB_FWI2D_PLAIN | GB_FWI2D_CHECKPOINT | GB_FWI2D_EXACT_GRADIENT | GB_FWI2D_GRAPH));

@@ -297,14 +297,12 @@ GBX_HD float div2_any(float x, float y, float r, int fast)
     return div_const2(x, y, r, fast);
 }
 
-GBX_COLD float div2_any_cold(float x, float y, float r, int fast) { return div2_any(x, y, r, fast); }
-
 // xs / y for a scaled dividend xs = x * 2^64 (|x| < 1, div_two_least(y) <= 2^-85:
-// x = +-0 or |xs| >= 2^-85), rounded as the float x / y is and scaled alike: q = RN(xs / y) where x / y is
-// normal, |q| >= 2^-62; below that the quotient rounded to the subnormal grid
-// G = 2^-149 * 2^64.  There (|q| + c) - c rounds |q| to even on G, the ulp of
-// [c, 2c); that is the rounding of the true quotient unless q is a midpoint by
-// its own rounding, and then the sign of the remainder decides.
+// x = +-0 or |xs| >= 2^-85), rounded as the float x / y is and scaled alike: q =
+// RN(xs / y) where x / y is normal, |q| >= 2^-62; below that the quotient rounded
+// to the subnormal grid G = 2^-149 * 2^64.  There (|q| + c) - c rounds |q| to even
+// on G, the ulp of [c, 2c); that is the rounding of the true quotient unless q is a
+// midpoint by its own rounding, and then the sign of the remainder decides.
 GBX_HD float div_two_tiny(float xs, float y, float rh, float rl)
 {
     const float q = div_two(xs, rh, rl), aq = std::fabs(q);

@@ -9,8 +9,8 @@
 // (:1053-1066) become a rotation of three buffers, so no step copies a field.
 //
 // The step kernels are in fwi2d_step.cuh; this file holds what they share
-// with the other kernels: the geometry, the buffers of a wave, the exact
-// boundary mix and the TMA / mbarrier helpers.
+// with the other kernels: the geometry, the buffers of a wave and the exact
+// boundary mix (the TMA and mbarrier helpers are in tma.cuh).
 //
 // Arithmetic of the forward pass follows the reference operation by
 // operation: __fmul_rn / __fadd_rn / __fsub_rn never contract into FMA;

@@ -42,9 +42,11 @@
 // step of 18 M padded cells): 112 with 32x16 tiles in one class and inline exact
 // fallbacks; 97 with the second differences' quotients in two operations and
 // the strips' and interior rows' loops separate; 81 with straight-line tails
-// and untouched tiles skipped; 76 with the tails out of line (no spills); 70 with
-// a shorter prologue.  Two columns a lane: 115 -> 70 instructions per 32 interior
-// cells (adjoint).
+// and untouched tiles skipped; 76 with the tails out of line (no spills in order
+// 8; the other orders' forward kernels spill 24 to 80 bytes under the cap of 72
+// registers, k_step_multi up to 224); 70 with a shorter prologue; 71.6 -> 74.4 with
+// the adjoint's boundary mix proved and its skipped tiles' stored field looked at.
+// Two columns a lane: 115 -> 70 instructions per 32 interior cells (adjoint).
 #pragma once
 
 #include "fwi2d_step_launch.h"

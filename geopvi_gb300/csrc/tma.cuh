@@ -74,14 +74,14 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, u
         : "memory");
 }
 
-// Bounded wait: true once phase `parity` completed, false after the limit
-// (the caller records the timeout and skips its work).
 // Programmatic dependent launch: wait for the previous grid on the stream
 // (complete, its writes visible), and let the next one be scheduled.  Both
 // are no-ops in a launch without the programmatic-serialization attribute.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Bounded wait: true once phase `parity` completed, false after the limit
+// (the caller records the timeout and skips its work).
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity)
 {
     for (int i = 0; i < (1 << 24); ++i)
